@@ -4,7 +4,7 @@ Every case goes through the public entry points (``ops``, ``w4a16``, ``chain``) 
 eagerly, or -- ``graph: True`` -- as a step captured once with ``timing.capture`` and replayed, which is how a decode
 loop runs.  A pass walks several layers' weights where one layer's would stay in the 126 MB L2 of the previous pass.
 
-``listed()`` are the fixed cases, ``draw(rng)`` one more of the same ranges.
+``listed()`` are the fixed cases, ``draw(rng)`` one more of the same ranges, ``exact`` the results in 64-bit arithmetic.
 """
 
 from __future__ import annotations
@@ -243,3 +243,86 @@ def tolerance(case: dict):
         return {"rel": 1e-2}
     dtype = case.get("dtype", "f16")
     return {"rel": {"f32": 1e-5 if kind == "attend" else 2e-6, "f16": 1e-3, "bf16": 7e-3}[dtype]}
+
+
+def _norm64(x, residual, weight):
+    s = x + residual
+    return s / (s.square().mean(-1, keepdim=True) + _EPS).sqrt() * weight, s
+
+
+def _int4_64(x, packed, scales, bias, group):
+    """x [M, K] times the weights the format defines: half(q * scale), low nibble first."""
+    k = x.shape[1]
+    codes = torch.stack((packed & 15, packed >> 4), dim=2).flatten(1)[:, :k].float() - 8
+    w = (codes * scales.float().repeat_interleave(group, dim=1)[:, :k]).half()
+    y = x @ w.double().t()
+    return y if bias is None else y + bias.double()
+
+
+def _rotate64(x, cos, sin, rope, interleaved):
+    """The first ``rope`` dims of each head of x [tokens, heads, dim] turned by the angles of cos, sin [tokens, rope / 2]."""
+    out, half = x.clone(), rope // 2
+    one, two = (slice(0, rope, 2), slice(1, rope, 2)) if interleaved else (slice(0, half), slice(half, rope))
+    a, b, c, s = x[..., one], x[..., two], cos.double()[:, None, :half], sin.double()[:, None, :half]
+    out[..., one], out[..., two] = a * c - b * s, a * s + b * c
+    return out
+
+
+def _slots(positions, page_table, sequence_ids, page):
+    return page_table[sequence_ids, positions // page], positions % page
+
+
+def _attend64(q, k_cache, v_cache, positions, page_table, sequence_ids, page, layout):
+    out = torch.empty_like(q, dtype=torch.float64)
+    for t in range(q.shape[0]):
+        js = torch.arange(int(positions[t]) + 1, device=q.device)
+        pages, offs = _slots(js, page_table, sequence_ids[t].expand(js.numel()), page)
+        k, v = ((c[pages, offs] if layout == "NHD" else c[pages, :, offs]).double() for c in (k_cache, v_cache))
+        heads = q[t].double().reshape(k.shape[1], -1, q.shape[2])  # [kv_heads, group, dim]
+        p = torch.softmax(torch.einsum("hgd,jhd->hgj", heads, k) * q.shape[2] ** -0.5, dim=-1)
+        out[t] = torch.einsum("hgj,jhd->hgd", p, v).reshape(q.shape[1:])
+    return out
+
+
+def exact(case: dict, seed: int):
+    """What ``run`` returns for these inputs, every operation in 64 bits and nothing rounded between them."""
+    kind = case["kind"]
+    st = prepare(dict(case, graph=False), seed)
+    if kind == "norm":
+        return _norm64(st["x"].double(), st["residual"].double(), st["weight"].double())
+    if kind == "linear":
+        ws = (w if case["layout"] == "KN" else w.t() for w in st["weights"])
+        return [st["x"].double() @ w.double() + b.double() for w, b in zip(ws, st["biases"])]
+    if kind == "int4":
+        return [_int4_64(st["x"].double(), p, s, b, case["group"]) for p, s, b in zip(st["packed"], st["scales"], st["biases"])]
+    if kind == "append":
+        pos, rope = st["positions"], case["rope_dim"]
+        pages, offs = _slots(pos, st["page_table"], st["sequence_ids"], case["page_size"])
+        at = (pages, offs) if case["layout"] == "NHD" else (pages, slice(None), offs)
+        turn = [_rotate64(st[n].double(), st["cos"][pos], st["sin"][pos], rope, case["interleaved"]) for n in ("q", "k")]
+        k_cache, v_cache = st["k_cache"].double(), st["v_cache"].double()
+        k_cache[at], v_cache[at] = turn[1], st["v"].double()
+        return turn[0], k_cache, v_cache
+    if kind == "attend":
+        return _attend64(st["q"], st["k_cache"], st["v_cache"], st["positions"], st["page_table"], st["sequence_ids"],
+                         case["page_size"], case["layout"])
+    chain, c = st["chain"], _config(case)
+    pos, table, seqs = (chain.dev[n] for n in ("positions", "page_table", "sequence_ids"))
+    k_cache, v_cache = chain.k_cache.double(), chain.v_cache.double()
+    at = _slots(pos, table, seqs, c.page_size)
+    h, res, out = chain.dev["h"].double(), chain.dev["res"].double(), {}
+    for layer in chain.layers:
+        n1, r1 = _norm64(h, res, layer["w1"].double())
+        qkv = _int4_64(n1, layer["qkv_packed"], layer["qkv_scales"], None, c.group)
+        heads = qkv.view(c.tokens, -1, c.head_dim)
+        cos, sin = chain.dev["cos"][pos], chain.dev["sin"][pos]
+        q_rot = _rotate64(heads[:, :c.q_heads], cos, sin, c.head_dim, False)
+        k_cache[at] = _rotate64(heads[:, c.q_heads:c.q_heads + c.kv_heads], cos, sin, c.head_dim, False)
+        v_cache[at] = heads[:, c.q_heads + c.kv_heads:]
+        attn = _attend64(q_rot, k_cache, v_cache, pos, table, seqs, c.page_size, "NHD").view(c.tokens, c.hidden)
+        n2, r2 = _norm64(attn, r1, layer["w2"].double())
+        up = _int4_64(n2, layer["up_packed"], layer["up_scales"], None, c.group)
+        act = torch.nn.functional.silu(up[:, c.mlp:]) * up[:, :c.mlp]
+        out = dict(n1=n1, r1=r1, qkv=qkv, q_rot=q_rot, attn=attn, n2=n2, r2=r2, up=up, up_all=up, act=act)
+        h, res = n2, r2
+    return {**out, "k_cache": k_cache, "v_cache": v_cache}
