@@ -11,6 +11,7 @@ import functools
 import pathlib
 
 LIB_PATH = pathlib.Path(__file__).resolve().parent / "libxdk_b200.so"
+HOST_PATH = LIB_PATH.with_name("_host.so")
 
 XDK_F32, XDK_BF16, XDK_F16 = 0, 1, 2
 XDK_STRICT_FP32, XDK_DEPENDENT_LAUNCH = 1, 2  # flags of the *_v2 entry points
@@ -86,6 +87,24 @@ def lib() -> ctypes.CDLL:
         fn.restype = restype
         fn.argtypes = argtypes
     return handle
+
+
+@functools.lru_cache(maxsize=1)
+def host():
+    """The native half of the ops (csrc/host.cpp): each function launches an ordinary call, or returns None."""
+    import importlib.machinery
+    import importlib.util
+
+    import torch  # noqa: F401  (its libraries first: the extension links against them)
+
+    if not HOST_PATH.exists():
+        raise NativeLibraryError(f"{HOST_PATH} is not built; run `python -m cross_dsl_kernels_b200.build`")
+    lib()
+    loader = importlib.machinery.ExtensionFileLoader("_host", str(HOST_PATH))
+    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_host", str(HOST_PATH), loader=loader))
+    loader.exec_module(module)
+    module.set_check(check)
+    return module
 
 
 def check(status: int, what: str) -> None:

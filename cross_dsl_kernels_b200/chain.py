@@ -215,9 +215,7 @@ class DecodeLayerChain:
         res = dv["res"] if res is None else res
         n1, r1 = fused_residual_rmsnorm(h, res, L["w1"], c.eps, dependent_launch=dep)
         qkv = w4a16_linear(n1, L["qkv_packed"], L["qkv_scales"], None, group_size=c.group, dependent_launch=dep)
-        q = qkv[:, : hq * d].view(c.tokens, hq, d)
-        k = qkv[:, hq * d: (hq + hkv) * d].view(c.tokens, hkv, d)
-        v = qkv[:, (hq + hkv) * d:].view(c.tokens, hkv, d)
+        q, k, v = qkv.view(c.tokens, hq + 2 * hkv, d).split((hq, hkv, hkv), dim=1)
         q_dst = self.q_peer[layer % 2] if peer else None
         sharded_attention = peer and self.attention
         q_rot = rope_gqa_paged_kv_append(q, k, v, dv["cos"], dv["sin"], dv["positions"], dv["page_table"],

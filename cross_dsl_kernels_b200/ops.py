@@ -14,6 +14,10 @@ reference it stands in for, so ``functools.partial(op, *case["args"],
 Checks mirror upstream's native bindings (csrc/*/*_ext.cpp) and raise
 ValueError; the kernels run on the tensor's device, on torch's current stream,
 without synchronising, and are safe under CUDA-graph capture.
+
+An ordinary call is checked and launched in native code (csrc/host.cpp), at a
+fraction of what the same checks cost here; whatever that declines -- every
+call that is refused among it -- takes the Python path below.
 """
 
 from __future__ import annotations
@@ -50,6 +54,9 @@ def fused_residual_rmsnorm(x, residual, weight, eps, *, return_residual: bool = 
     ``dependent_launch=True`` (every op of this module takes it) launches the kernel as a programmatic
     dependent of the preceding kernel on the stream, so that its scheduling and set-up overlap that
     kernel's tail; the caller promises that ``weight`` was not written by that kernel."""
+    done = _native.host().rmsnorm(x, residual, weight, eps, return_residual, dependent_launch)
+    if done is not None:
+        return done
     _gate(x)
     _need(residual.is_cuda and weight.is_cuda, "residual and weight must be CUDA tensors")
     _need(x.dtype in _RMS_DTYPES, "x must be float32, bfloat16 or float16")
@@ -86,6 +93,10 @@ def decode_linear(x, weight, bias=None, *, out_dtype=None, weight_layout: str = 
     ``peer_out`` (multi-GPU; from :meth:`cross_dsl_kernels_b200.peer.PeerMatrix.out_for`): the kernel stores its
     [M, N] result into columns [col0, col0 + N) of the full-width matrix on every rank instead of allocating
     an output; the call then returns None and the caller orders readers with ``PeerArena.barrier``."""
+    if peer_out is None and out_dtype is None and strict_fp32 is False:
+        done = _native.host().linear(x, weight, bias, weight_layout, split_k, dependent_launch)
+        if done is not None:
+            return done
     _need(x.dim() == 2, "x must be a 2D tensor shaped [M, K]")
     _need(weight.dim() == 2, "weight must be a 2D tensor")
     _need(weight_layout in ("KN", "NK"), "weight_layout must be 'KN' or 'NK'")
@@ -140,6 +151,11 @@ def rope_gqa_paged_kv_append(q, k, v, cos, sin, positions, page_table, sequence_
     Index values are trusted: validate them once at set-up with
     :func:`cross_dsl_kernels_b200.references.validate_paged_kv_indices`.
     """
+    if q_peer_out is None:
+        done = _native.host().append(q, k, v, cos, sin, positions, page_table, sequence_ids, k_cache, v_cache, page_size, rope_dim,
+                                     interleaved, kv_layout, dependent_launch)
+        if done is not None:
+            return done
     _gate(q)
     dtype = q.dtype
     _need(dtype in _RMS_DTYPES, "q must be float32, bfloat16 or float16")
@@ -209,6 +225,11 @@ def paged_decode_attention(q, k_cache, v_cache, positions, page_table, sequence_
     ``peer_out`` (multi-GPU; :meth:`cross_dsl_kernels_b200.peer.PeerMatrix.out_for`): the result goes to columns
     [col0, col0 + q_heads * head_dim) of every rank's copy of a [tokens, all heads * head_dim] matrix instead of a
     fresh tensor, and the call returns None; readers wait for the arena's flag barrier."""
+    if peer_out is None:
+        done = _native.host().attention(q, k_cache, v_cache, positions, page_table, sequence_ids, page_size, kv_layout, scale,
+                                        context_hint, dependent_launch)
+        if done is not None:
+            return done
     _gate(q)
     dtype = q.dtype
     _need(dtype in _RMS_DTYPES, "q must be float32, bfloat16 or float16")
@@ -252,6 +273,10 @@ def swiglu(upgate, *, dependent_launch: bool = False, peer_out=None):
     """silu(gate) * up for a fused projection output ``[rows, 2 * width]`` laid out [up | gate]; returns [rows, width].
     Rows may be a fixed number of elements apart (a column slice of a wider matrix).  Not part of upstream.
     ``peer_out``: as for :func:`paged_decode_attention` (columns [col0, col0 + width) of every rank's matrix)."""
+    if peer_out is None:
+        done = _native.host().swiglu(upgate, dependent_launch)
+        if done is not None:
+            return done
     _gate(upgate)
     _need(upgate.dtype in _RMS_DTYPES, "upgate must be float32, bfloat16 or float16")
     _need(upgate.dim() == 2 and upgate.shape[1] % 2 == 0 and upgate.shape[0] > 0 and upgate.shape[1] > 0,

@@ -48,6 +48,10 @@ def w4a16_linear(x, packed, scales, bias=None, *, group_size=128, backend="cuda"
     packed codes, scales and bias must not be that kernel's output; ``x`` may be).  ``peer_out`` (multi-GPU, from
     ``PeerMatrix.out_for``): store the result into this rank's columns of the full-width matrix on every rank;
     nothing is allocated and None is returned."""
+    if backend == "cuda" and peer_out is None and type(rows_per_block) is int and rows_per_block in (1, 4):
+        done = _native.host().w4a16(x, packed, scales, bias, group_size, out, dependent_launch)
+        if done is not None:
+            return done
     if backend != "cuda":
         if backend in ("reference", "triton", "cute"):
             raise ValueError(f"backend {backend!r} is not part of this library: it runs the sm_100a CUDA kernel only")
