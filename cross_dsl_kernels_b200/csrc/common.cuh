@@ -36,6 +36,9 @@ unsigned w4a16_fault_word();
 bool gemv_tc_eligible(const float* x, const float* w, int64_t m, int64_t k, int64_t n, bool nk);
 int gemv_tc_plan(int64_t m, int64_t k, int64_t n, bool nk, int32_t out[5]);  // {CTAs, lane-quarter K split, ring depth, smem bytes, units}; returns the cluster size, 0 = declined
 
+// FP32 projection of more than 16 rows on mma.sync (gemv_mma.cu): whether it takes the operands (its launch is below)
+bool gemv_mma_eligible(const float* x, const float* w, int64_t m, int64_t k, int64_t n, bool nk);
+
 // Flags of the *_v2 entry point that is executing on this host thread (0 outside one).
 unsigned call_flags();
 void set_call_flags(unsigned flags);
@@ -108,6 +111,8 @@ inline PeerOut single_out(void* y, int64_t ld) {
 // Copies and checks the caller's descriptor (NULL: `fallback` / `ld` as the only destination).
 int make_out(const xdk_peer_out* peers, void* fallback, int64_t ld, PeerOut* out);
 unsigned peer_fault_word();
+int launch_gemv_mma(const float* x, const float* w, const float* bias, const PeerOut& y, int m, int k, int n, bool nk,
+                    cudaStream_t stream);
 int launch_gemv_tc(const float* x, const float* w, const float* bias, const PeerOut& y, int m, int k, int n, bool nk,
                    cudaStream_t stream);
 

@@ -733,6 +733,12 @@ extern "C" int xdk_gemv_f32_peer(const float* x, const float* w, const float* bi
   if (int st = require_sm100()) return st;
   const bool nk = weight_is_nk != 0;
 
+  // More than 16 rows unless strict FP32 was asked for: the mma.sync split-TF32 kernel (gemv_mma.cu, with both sides' times
+  // and errors).  It would also be faster than the tcgen05 kernel for 5 .. 8 rows of a wide [K, N] matrix (N = 11012 41 us
+  // against 50), but not for 16 (N = 14336 60 / 50), and a row keeps its bits whatever the batch of up to 16 it is in.
+  if (split_k == 0 && !strict && m > 16 && gemv_mma_eligible(x, w, m, k, n, nk))
+    return launch_gemv_mma(x, w, bias, y, static_cast<int>(m), static_cast<int>(k), static_cast<int>(n), nk, static_cast<cudaStream_t>(stream));
+
   // 4 < M <= 16 unless strict FP32 was asked for: the tcgen05 kernel (split-TF32 products, FP32 accumulation; see
   // gemv_tc.cu).  Everything below this line is FP32 FMA arithmetic.
   if (split_k == 0 && !strict && gemv_tc_eligible(x, w, m, k, n, nk))
