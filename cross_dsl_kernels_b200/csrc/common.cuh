@@ -135,6 +135,13 @@ __device__ __forceinline__ U4 ld_cached16(const void* p) {
   const uint4 t = __ldg(reinterpret_cast<const uint4*>(p));
   return U4{t.x, t.y, t.z, t.w};
 }
+// 128-bit load of what the preceding kernel wrote.  Volatile, so that it stays behind pdl_wait(): a load through the
+// read-only path (ld_cached16) counts as invariant and the compiler may move it in front of the wait.
+__device__ __forceinline__ U4 ld_ordered16(const void* p) {
+  U4 v;
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
 __device__ __forceinline__ float4 ld_stream_f4(const float* p) {
   float4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];"

@@ -9,16 +9,20 @@
 // that FP32 product is exact.  Products with x accumulate in FP32.
 //
 // Compute paths (they share the unpack; the dispatcher at the end of the file picks one):
-//   * M <= 8, K % 1024 == 0: mma.m16n8k16 with the operands swapped -- 16 weight columns are the MMA's rows, the rows of
+//   * small M, K % 1024 == 0: mma.m16n8k16 with the operands swapped -- 16 weight columns are the MMA's rows, the rows of
 //     x its columns -- fed from direct 16-byte loads (w4a16_mma_kernel).
-//   * M >= 9 (and any M with a strided or multi-rank output), K % 256 == 0, group >= 64: tcgen05 kind::f16 with the
-//     dequantised weights in tensor memory (w4a16_umma_kernel).
-//   * shapes those two decline: a TMA-fed mma.sync stream kernel (M >= 3, K % 128 == 0), a SIMT kernel (lanes stride
-//     over the packed row, mixed-precision FMAs, warp shuffle per column) and a generic kernel for any K.
+//   * M >= 9 on widths that suit its strips (and any M with a strided or multi-rank output), K % 256 == 0, group >= 64:
+//     tcgen05 kind::f16 with the dequantised weights in tensor memory (w4a16_umma_kernel).
+//   * the other M >= 3, K % 128 == 0: the same MMAs with x kept in registers and K shared by the warps of a CTA or the
+//     CTAs of a cluster (w4a16_rx_kernel).
+//   * the rest: a TMA-fed mma.sync stream kernel (K > 32768), a SIMT kernel (lanes stride over the packed row,
+//     mixed-precision FMAs, warp shuffle per column) and a generic kernel for any K.
 // The k order inside an MMA fragment is free as long as both operands use the same order, so x is stored in shared
 // memory pre-permuted to the order the unpack produces and no weight ever moves between lanes.
 #include <cooperative_groups.h>
 #include <stdlib.h>
+
+#include <atomic>
 
 #include "common.cuh"
 #include "umma.cuh"
@@ -182,7 +186,7 @@ __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1
 __device__ __forceinline__ int xunit(int unit, int row) { return unit ^ ((((unit >> 3) & 1) << 1) | (row & 1)); }
 
 // ------------------------------------------------------------------------------------------------
-// Streaming tensor-core path (the one used for 3 <= M <= 16 when K % 128 == 0).
+// Streaming tensor-core path (M >= 3, K % 128 == 0, K too long for the paths below).
 //
 // One persistent CTA per SM.  The N/8 column blocks are dealt out evenly to clusters of S CTAs
 // (S = split-K factor, 1/2/4); inside a cluster CTA r takes the K chunks r, r+S, ... of 1024 k, and
@@ -980,9 +984,9 @@ w4a16_generic_kernel(W4Args a) {
 // are simply "the pairs the unpack produces": word w of a vector gives A pairs (k0,k4) (k1,k5) for one MMA and
 // (k2,k6) (k3,k7) for the next, and the matching B pairs are one 16-byte read of x, which sits in shared memory
 // already permuted to (0,4,1,5,2,6,3,7) inside every 8 k.  The legacy HMMA pipe of this part retires one m16n8k16
-// per 32 cycles and sub-partition (6.3 us for K = 4096, N = 14336 in this form; with x as the 16-row operand it
-// would be twice that), so the rest of the instruction stream has to fit beside it: 26 warp instructions per MMA
-// are left (13 of them the exact unpack), after taking everything out of the loop that does not depend on the
+// per 8 cycles and sub-partition (measured; 1.6 us for K = 4096, N = 14336 in this form), the 13 instructions of the exact
+// unpack take 24, so the instruction stream is what counts: 26 warp instructions per MMA
+// are left, after taking everything out of the loop that does not depend on the
 // codes -- no zero-filling of registers for columns past N or rows past M (they read a valid column or row and
 // feed outputs that are never stored), scales widened to half2 when they are fetched, one base pointer per column.
 // The grid is one wave (as many CTAs as are resident at once), the groups of 16 columns dealt evenly.
@@ -1132,6 +1136,313 @@ int launch_mma(W4Args a, bool dependent, cudaStream_t stream) {
   return launch_opts(w4a16_mma_kernel, dim3(ctas), dim3(kThreads), smem, stream, 1u, dependent, a, groups);
 }
 
+// ------------------------------------------------------------------------------------------------
+// Tensor-core path for K % 128 == 0 (every M, every group size): x stays in registers, W streams past it.
+//
+// An MMA (m16n8k16) takes 16 columns of W as its rows and 8 rows of x as its columns.  A warp owns one slice of 256 k
+// and keeps x of that slice -- all rows -- in registers as ready B fragments (32 registers per 8 rows); it walks
+// column groups of 16, one pass each.  So the loop touches shared memory only for the codes: TMA box copies
+// ([16 columns][128 B], 128-byte swizzle) into a ring private to the warp, refilled by the warp itself.  Lane
+// (i = lane / 4, q = lane % 4) unpacks 32 codes of two columns at a time; the slots of a fragment are simply "the half2
+// pairs the exact unpack produces": word w of a vector gives A pairs (k0,k4) (k1,k5) for one MMA and (k2,k6) (k3,k7)
+// for the next, and x is permuted to match when it is loaded.  MMA row i stands for column (i / 2) + 4 (i % 2) of the
+// group: with the swizzle, the two rows a quarter-warp reads then lie on different halves of the banks.
+//
+// The warps of a column set (one per slice) park their partial sums in shared memory, pass by pass; the warp whose turn
+// it is adds them in slice order one pass later, so nobody waits at a barrier.  K > 4096 is split over the CTAs of a
+// cluster: a rank's sums go through distributed shared memory to the rank that owns the pass, and are added there, in
+// rank order, once after the cluster's barrier.  K < 4096 leaves warps over, which form further column sets.
+//
+// What bounds it: the exact unpack.  HFMA2 and LOP3 take two issue slots each and do not overlap on this part, so the 13
+// instructions of eight codes cost a sub-partition 24 cycles per 256 weights, an MMA 8 (measured); a pass runs at about
+// half of that bound, the rest is the passes' hand-overs.  Against the tcgen05 kernel, which pays for K split over its lane
+// quarters with four x ranges a step: M = 16, K = 14336, N = 4096 34.0 -> 22.6 us, K = 11008 30.5 -> 19.6; the dispatch at the
+// end of the file has both sides of its rule.  The lanes sharing one scale load each through shuffles measured slower
+// (M = 1, N = 28672 25.6 against 22.7).
+constexpr int kRxWarps = 16;       // at most, per CTA (one CTA per SM: 128 registers a thread)
+constexpr int kRxSliceK = 256;     // k per warp
+constexpr int kRxStage = 16 * kRxSliceK / 2;  // bytes of codes of a pass
+constexpr int kRxMaxDepth = 6;     // passes in flight per warp
+constexpr int kRxParts = 3;        // buffers of partial sums per column set
+constexpr int kRxMaxPasses = 64;   // of a cluster: bounds the sums it parks
+constexpr int kRxSmem = 226 * 1024;
+
+struct RxPlan {
+  int slices;      // of K, all ranks
+  int ranks;       // CTAs per cluster that share K
+  int cta_slices;  // slices per CTA
+  int sets;        // column sets per CTA
+  int total_sets;  // of the launch
+  int groups;      // column groups of 16
+  int depth;       // ring slots per warp
+  int parked;      // passes a rank owns (ranks > 1)
+};
+
+template <int MR>  // rows of x in eights
+__global__ void __launch_bounds__(kRxWarps * 32, 1)
+w4a16_rx_kernel(W4Args a, RxPlan plan, const __grid_constant__ CUtensorMap wmap) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  const int warps = plan.cta_slices * plan.sets;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = lane >> 2, q = lane & 3;
+  const int set = warp / plan.cta_slices, ws = warp - set * plan.cta_slices;
+  const int rank = blockIdx.y;
+  const int slice = rank * plan.cta_slices + ws;
+  const int live_slices = min(plan.cta_slices, plan.slices - rank * plan.cta_slices);  // the last rank may hold fewer
+  const int depth = plan.depth;
+  unsigned char* ring = smem_raw + warp * depth * kRxStage;
+  float4* part = reinterpret_cast<float4*>(smem_raw + warps * depth * kRxStage) + set * kRxParts * plan.cta_slices * MR * 32;
+  float4* parked = reinterpret_cast<float4*>(smem_raw + warps * depth * kRxStage) + plan.sets * kRxParts * plan.cta_slices * MR * 32;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(parked + (plan.ranks > 1 ? plan.parked * plan.ranks * MR * 32 : 0));
+  uint64_t* full = bars + warp * depth;                                  // this warp's slots
+  uint64_t* part_full = bars + warps * depth + set * 2 * kRxParts;       // every warp of the set wrote its partial sums
+  uint64_t* part_empty = part_full + kRxParts;                           // they have been added
+
+  const int set_id = blockIdx.x * plan.sets + set;
+  const int g0 = static_cast<int>(static_cast<int64_t>(set_id) * plan.groups / plan.total_sets);
+  const int passes = ws < live_slices
+      ? static_cast<int>(static_cast<int64_t>(set_id + 1) * plan.groups / plan.total_sets) - g0 : 0;
+
+  auto issue = [&](int slot, int pass) {  // one lane
+    mbar_expect_tx(full + slot, kRxStage);  // parts of a box past K or N are zero-filled and still counted
+    tma_box_2d(ring + slot * kRxStage, &wmap, slice * (kRxSliceK / 8), (g0 + pass) * 16, full + slot);
+  };
+  if (lane == 0) {
+    for (int s = 0; s < depth; ++s) mbar_init(full + s, 1);
+    if (ws == 0)
+      for (int b = 0; b < kRxParts; ++b) mbar_init(part_full + b, live_slices), mbar_init(part_empty + b, 1);
+    mbar_fence_init();
+    for (int p = 0; p < depth && p < passes; ++p) issue(p, p);  // the weights do not depend on the preceding kernel
+    pdl_launch_dependents();
+  }
+  const int col_lo = (i >> 1) + ((i & 1) << 2);  // this lane's columns of a group: col_lo and col_lo + 8
+  const int k0 = slice * kRxSliceK + q * 32;
+  // this lane's scales of a pass, fetched a pass ahead: two columns h, its quarter of each 128-k chunk c
+  const int scale_shift = 31 - __clz(a.group);
+  int scale_idx[2];
+#pragma unroll
+  for (int c = 0; c < 2; ++c) scale_idx[c] = min((k0 + c * 128) >> scale_shift, a.groups - 1);  // past K: any, x is zero there
+  __half scale_next[2][2];
+  auto fetch_scales = [&](int pass) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {  // past N: any column, its sums are not stored
+      const __half* at = a.scales + static_cast<size_t>(min((g0 + pass) * 16 + h * 8 + col_lo, a.n - 1)) * a.groups;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) scale_next[c][h] = __ldg(at + scale_idx[c]);
+    }
+  };
+  fetch_scales(0);
+  __syncthreads();  // barriers of the sets
+  if (plan.ranks > 1) cg::this_cluster().barrier_arrive();  // the other ranks' shared memory is there after the wait
+
+  pdl_wait();  // x may be the preceding kernel's output; codes, scales and bias are not
+  uint32_t xf[2][MR][4][4];  // [chunk of 128 k][row group][word][fragment pair]
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int r = 0; r < MR; ++r) {
+      // rows past M and k past K are zeros; they read a valid address, so that the loads go out without a branch
+      const int row = r * 8 + i, k = k0 + c * 128;
+      const bool live = row < a.m && k < a.k;
+      const __half* src = a.x + static_cast<size_t>(min(row, a.m - 1)) * a.k + (k < a.k ? k : 0);
+      U4 v[4];
+#pragma unroll
+      for (int w = 0; w < 4; ++w) v[w] = ld_ordered16(src + w * 8);
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {  // k 0..7 -> 0,4 1,5 2,6 3,7
+        xf[c][r][w][0] = live ? __byte_perm(v[w].x, v[w].z, 0x5410) : 0u;
+        xf[c][r][w][1] = live ? __byte_perm(v[w].x, v[w].z, 0x7632) : 0u;
+        xf[c][r][w][2] = live ? __byte_perm(v[w].y, v[w].w, 0x5410) : 0u;
+        xf[c][r][w][3] = live ? __byte_perm(v[w].y, v[w].w, 0x7632) : 0u;
+      }
+    }
+  if (plan.ranks > 1) cg::this_cluster().barrier_wait();
+
+  bool ok = true;
+  const size_t out_at = static_cast<size_t>(q * 2) * a.out.ld + a.out.col0 + g0 * 16 + col_lo;
+  auto store = [&](int pass, const float4 (&sum)[MR]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int col = (g0 + pass) * 16 + h * 8 + col_lo;
+      if (col >= a.n) continue;
+      const float bv = a.bias ? __half2float(a.bias[col]) : 0.0f;
+      for (int p = 0; p < a.out.world; ++p) {
+        __half* dst = static_cast<__half*>(a.out.ptr[p]) + out_at + pass * 16 + h * 8;
+#pragma unroll
+        for (int r = 0; r < MR; ++r) {
+          if (r * 8 + q * 2 < a.m) dst[r * 8 * a.out.ld] = __float2half_rn((h ? sum[r].z : sum[r].x) + bv);
+          if (r * 8 + q * 2 + 1 < a.m) dst[(r * 8 + 1) * a.out.ld] = __float2half_rn((h ? sum[r].w : sum[r].y) + bv);
+        }
+      }
+    }
+  };
+  auto reduce = [&](int pass) {  // one warp: the partial sums of a pass in slice order
+    const int b = pass % kRxParts;
+    if (ok) ok = mbar_wait(part_full + b, (pass / kRxParts) & 1);
+    const float4* src = part + b * plan.cta_slices * MR * 32 + lane;
+    float4 sum[MR];
+#pragma unroll
+    for (int r = 0; r < MR; ++r) sum[r] = src[r * 32];
+#pragma unroll 4
+    for (int s = 1; s < live_slices; ++s)
+#pragma unroll
+      for (int r = 0; r < MR; ++r) {
+        const float4 v = src[(s * MR + r) * 32];
+        sum[r].x = __fadd_rn(sum[r].x, v.x), sum[r].y = __fadd_rn(sum[r].y, v.y);
+        sum[r].z = __fadd_rn(sum[r].z, v.z), sum[r].w = __fadd_rn(sum[r].w, v.w);
+      }
+    __syncwarp();
+    if (lane == 0) mbar_arrive_cta(part_empty + b);
+    if (plan.ranks == 1) {
+      if (ok) store(pass, sum);
+    } else {
+      const int owner = pass % plan.ranks;
+      const uint32_t dst = cluster_map(parked + ((pass / plan.ranks) * plan.ranks + rank) * MR * 32 + lane, owner);
+#pragma unroll
+      for (int r = 0; r < MR; ++r) cluster_store_f4(dst + r * 32 * sizeof(float4), sum[r]);
+    }
+  };
+
+  RingPos slot, pb;  // ring slot, partial-sum buffer
+  int turn = 0;      // whose turn it is to add the previous pass (pass - 1) % live_slices
+  for (int pass = 0; pass < passes; ++pass) {
+    __half2 sc[2][2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) sc[c][h] = __half2half2(scale_next[c][h]);
+    if (pass + 1 < passes) fetch_scales(pass + 1);
+    if (ok) ok = mbar_wait(full + slot.slot, slot.parity);
+    float acc[MR][4];
+#pragma unroll
+    for (int r = 0; r < MR; ++r)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[r][e] = 0.0f;
+    const unsigned char* lo = ring + slot.slot * kRxStage + col_lo * 128;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int at = ((c * 4 + q) ^ col_lo) << 4;
+      const U4 v0 = *reinterpret_cast<const U4*>(lo + at), v1 = *reinterpret_cast<const U4*>(lo + 8 * 128 + at);
+      const uint32_t w0[4] = {v0.x, v0.y, v0.z, v0.w}, w1[4] = {v1.x, v1.y, v1.z, v1.w};
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        __half2 h0[4], h1[4];
+        dequant8(w0[w], sc[c][0], h0);
+        dequant8(w1[w], sc[c][1], h1);
+        const uint32_t* f0 = reinterpret_cast<const uint32_t*>(h0);
+        const uint32_t* f1 = reinterpret_cast<const uint32_t*>(h1);
+#pragma unroll
+        for (int r = 0; r < MR; ++r) mma16816(acc[r], f0[0], f1[0], f0[1], f1[1], xf[c][r][w][0], xf[c][r][w][1]);
+#pragma unroll
+        for (int r = 0; r < MR; ++r) mma16816(acc[r], f0[2], f1[2], f0[3], f1[3], xf[c][r][w][2], xf[c][r][w][3]);
+      }
+    }
+    __syncwarp();  // every lane has read the slot
+    if (lane == 0 && pass + depth < passes) issue(slot.slot, pass + depth);
+    slot.advance(depth);
+    if (ok) ok = mbar_wait(part_empty + pb.slot, pb.parity ^ 1u);  // a fresh barrier passes: nothing is parked yet
+    float4* mine = part + (pb.slot * plan.cta_slices + ws) * MR * 32 + lane;
+#pragma unroll
+    for (int r = 0; r < MR; ++r) mine[r * 32] = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+    __syncwarp();
+    if (lane == 0) mbar_arrive_cta(part_full + pb.slot);
+    pb.advance(kRxParts);
+    if (pass > 0) {
+      if (ws == turn) reduce(pass - 1);
+      if (++turn == live_slices) turn = 0;
+    }
+  }
+  if (passes > 0 && ws == turn) reduce(passes - 1);
+  if (plan.ranks > 1) {
+    __syncwarp();
+    cg::this_cluster().barrier_arrive();  // release: the sums pushed to other ranks
+    cg::this_cluster().barrier_wait();
+    const int all = static_cast<int>(static_cast<int64_t>(set_id + 1) * plan.groups / plan.total_sets) - g0;
+    for (int p = warp * plan.ranks + rank; p < all; p += warps * plan.ranks) {
+      const float4* src = parked + (p / plan.ranks) * plan.ranks * MR * 32 + lane;
+      float4 sum[MR];
+#pragma unroll
+      for (int r = 0; r < MR; ++r) sum[r] = src[r * 32];
+      for (int s = 1; s < plan.ranks; ++s)
+#pragma unroll
+        for (int r = 0; r < MR; ++r) {
+          const float4 v = src[(s * MR + r) * 32];
+          sum[r].x = __fadd_rn(sum[r].x, v.x), sum[r].y = __fadd_rn(sum[r].y, v.y);
+          sum[r].z = __fadd_rn(sum[r].z, v.z), sum[r].w = __fadd_rn(sum[r].w, v.w);
+        }
+      store(p, sum);
+    }
+  }
+  if (!ok && lane == 0) atomicOr(&g_w4_fault, 2u);
+}
+
+// Clusters of `ranks` such CTAs (one per SM) that are resident at once on the current device.
+int rx_resident_clusters(int ranks) {  // the same for every variant: one CTA per SM
+  static std::atomic<int> known[64][9];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int n = known[dev][ranks].load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  if (cudaFuncSetAttribute(w4a16_rx_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRxSmem) != cudaSuccess) return 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(sm_count() / ranks, ranks);
+  cfg.blockDim = dim3(kRxWarps * 32);
+  cfg.dynamicSmemBytes = kRxSmem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1, attr[0].val.clusterDim.y = static_cast<unsigned>(ranks), attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr, cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, w4a16_rx_kernel<2>, &cfg) != cudaSuccess || n < 1) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  known[dev][ranks].store(n, std::memory_order_relaxed);
+  return n;
+}
+
+template <int MR>
+int launch_rx(const W4Args& a, bool dependent, cudaStream_t stream) {
+  RxPlan p = {};
+  cudaError_t err = cudaFuncSetAttribute(w4a16_rx_kernel<MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRxSmem);
+  if (err != cudaSuccess) return note_launch(err);
+  const int sms = sm_count();
+  p.slices = (a.k + kRxSliceK - 1) / kRxSliceK;
+  p.groups = (a.n + 15) / 16;
+  p.ranks = (p.slices + kRxWarps - 1) / kRxWarps;
+  // few columns: more CTAs share K, down to four slices each, while they all fit
+  while (p.ranks * 2 <= 8 && p.groups * p.ranks * 2 <= sms && p.slices >= p.ranks * 8) p.ranks *= 2;
+  if (p.ranks > 8) return XDK_ERR_LIMIT;
+  p.cta_slices = (p.slices + p.ranks - 1) / p.ranks;
+  p.ranks = (p.slices + p.cta_slices - 1) / p.cta_slices;
+  p.sets = 1;
+  int passes;
+  if (p.ranks == 1) {
+    p.sets = min(kRxWarps / p.cta_slices, (p.groups + sms - 1) / sms);
+    p.total_sets = min(sms, (p.groups + p.sets - 1) / p.sets) * p.sets;
+  } else {
+    int clusters = rx_resident_clusters(p.ranks);
+    if (clusters < 1) return XDK_ERR_LIMIT;
+    clusters = min(clusters, p.groups);
+    p.total_sets = max(clusters, (p.groups + kRxMaxPasses - 1) / kRxMaxPasses);
+  }
+  passes = (p.groups + p.total_sets - 1) / p.total_sets;
+  p.parked = p.ranks > 1 ? (passes + p.ranks - 1) / p.ranks : 0;
+  const int warps = p.cta_slices * p.sets;
+  const int fixed = (kRxParts * warps + p.parked * (p.ranks > 1 ? p.ranks : 0)) * MR * 512 +
+                    (warps * kRxMaxDepth + p.sets * 2 * kRxParts) * static_cast<int>(sizeof(uint64_t));
+  p.depth = min(min(kRxMaxDepth, passes), (kRxSmem - fixed) / (warps * kRxStage));
+  if (p.depth < 1) return XDK_ERR_LIMIT;
+  const size_t smem = static_cast<size_t>(fixed) + static_cast<size_t>(warps) * p.depth * kRxStage;
+  CUtensorMap wmap;
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(a.k / 8), static_cast<cuuint64_t>(a.n)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(a.k / 2)};
+  const cuuint32_t box[2] = {kRxSliceK / 8, 16};
+  static_assert(kRxSliceK / 2 == 128, "the box of codes is one 128-byte swizzle span wide");
+  if (!encode_tiled(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, a.packed, dims, strides, box, true)) return XDK_ERR_LAUNCH;
+  return launch_opts(w4a16_rx_kernel<MR>, dim3(p.total_sets / p.sets, p.ranks), dim3(warps * 32), smem, stream,
+                     static_cast<unsigned>(p.ranks), dependent, a, p, wmap);
+}
+
 template <int MT, int CW>
 int launch_simt(W4Args a, cudaStream_t stream) {
   const size_t smem = static_cast<size_t>(MT) * a.k * sizeof(__half);
@@ -1201,23 +1512,33 @@ extern "C" int xdk_w4a16_peer(const void* x, const uint8_t* packed, const void* 
   const bool dependent = (flags & XDK_DEPENDENT_LAUNCH) != 0;
   a.out = out;
   const bool vec_ok = k % 32 == 0 && aligned16(packed) && aligned16(x);  // 16-byte vectors of 32 codes
-  // M <= 8 with K a multiple of 1024 and x small enough for shared memory: the direct-load mma.sync kernel
-  // (K = 4096: N = 4096 5.9 / 6.0 / 6.4 / 7.2 us at M = 1 / 2 / 4 / 8, N = 14336 14.7 / 14.8 / 15.3 / 16.1, N = 28672
-  // 23.3 - 24.9; K = 14336, N = 4096: 13.9 / 14.6 / 19.9 at M = 1 / 2 / 4 -- against 6.4 / 16.3 / 30.1 / 17.3 at M = 1
-  // for the SIMT kernel and 10.2 - 10.8 / 16.6 - 17.0 / 28.5 - 29.2 / 21.5 - 25.8 for the tcgen05 kernel).
-  // XDK_W4A16_MMA=0 leaves these shapes to the kernels below (comparison runs).
+  // Who takes what, by measurement (us; K = 4096 unless said):
+  //  * M <= 2, K a multiple of 1024, and M <= 8 while x leaves room for two CTAs per SM: the direct-load mma.sync kernel
+  //    (N = 4096 6.0 / 6.5 / 7.3 at M = 1 / 4 / 8, N = 14336 14.7 / 15.7 / 16.4; the kernel that keeps x in registers 7.6 /
+  //    7.9 / 8.5 and 16.4 / 17.2 / 17.7; the SIMT kernel 16.3 at M = 1, N = 14336).
+  //  * M >= 9 where the tcgen05 kernel's CTAs walk whole strips, three or four 32-column units wide, or two of a short K:
+  //    the tcgen05 kernel (M = 16: N = 14336 17.6 against 20.8, N = 16384 17.7 / 21.2, N = 8192 13.9 / 14.5), and every
+  //    strided or multi-rank output.
+  //  * every other M >= 3: the kernel that keeps x in registers.  M = 16: one unit a CTA, i.e. K split over the lane
+  //    quarters (N = 2048 8.0 against 10.9, K = 14336, N = 4096 22.6 / 34.0, K = 11008 19.6 / 30.5), a strip and a narrow rest
+  //    (N = 24576 26.0 / 27.2), shapes the tcgen05 kernel declines (K = 2304, N = 8192 11.8 / 15.5); M = 8: x too large for two
+  //    CTAs (K = 14336, N = 4096 18.9 / 27.9, K = 7168, N = 20480 29.6 / 39.9), K = 2304, N = 8192 9.8 / 14.1.
+  // XDK_W4A16_MMA=0 and XDK_W4A16_UMMA=0 / 1 take the first kernel out, and the second out or in wherever it can run
+  // (comparison runs).
   static const bool mma_env = !(getenv("XDK_W4A16_MMA") && getenv("XDK_W4A16_MMA")[0] == '0');
-  if (mma_env && plain && vec_ok && m <= 8 && k % 1024 == 0 &&
-      static_cast<size_t>(m) * (static_cast<size_t>(k) * 2 + 16) <= 160 * 1024)
-    return launch_mma(a, dependent, s);
-  // M >= 9, smaller M where the kernel above does not apply (M >= 3, M = 2 on large matrices), and every M whose
-  // output is strided or goes to several ranks: the tcgen05 kernel.  Its time hardly depends on M (K = 4096,
-  // N = 14336: 17.1 us at M = 1, 17.6 at M = 8, 18.2 at M = 16).  XDK_W4A16_UMMA=0 keeps it for strided and
-  // multi-rank outputs only (comparison runs).
   static const int umma_env = getenv("XDK_W4A16_UMMA") ? (getenv("XDK_W4A16_UMMA")[0] == '1' ? 1 : 0) : -1;
+  const size_t x_bytes = static_cast<size_t>(m) * (static_cast<size_t>(k) * 2 + 16);
+  if (mma_env && plain && vec_ok && k % 1024 == 0 && (m <= 2 ? x_bytes <= 160 * 1024 : m <= 8 && x_bytes <= 104 * 1024))
+    return launch_mma(a, dependent, s);
   const bool umma_ok = vec_ok && k % 256 == 0 && group_size >= 64 && a.groups <= 256 && a.groups % 8 == 0 && aligned16(scales);
-  const int umma_min_m = k * n >= (32LL << 20) ? 2 : 3;
-  if (umma_ok && ((umma_env != 0 && m >= umma_min_m) || !plain)) {
+  const int64_t units = ((n + 31) / 32 + sm_count() - 1) / sm_count();  // 32-column units of the tcgen05 kernel's busiest CTA
+  const bool whole = units % 4 == 0 || units == 3 || (units == 2 && k < 8192) || (units > 4 && k > 4096);
+  const bool umma_first = !plain || umma_env == 1 || (m > 8 && whole && umma_env != 0);
+  if (plain && vec_ok && k % 128 == 0 && m >= 3 && !(umma_ok && umma_first)) {
+    const int st = m > 8 ? launch_rx<2>(a, dependent, s) : launch_rx<1>(a, dependent, s);
+    if (st != XDK_ERR_LIMIT) return st;  // K > 32768: the kernels below
+  }
+  if (umma_ok && (!plain || (umma_env != 0 && (m >= 3 || (m == 2 && k * n >= (32LL << 20)))))) {
     const int st = launch_umma(a, dependent, s);
     if (st != XDK_ERR_LIMIT || !plain) return st;
   }

@@ -1,0 +1,40 @@
+"""The W4A16 kernel that keeps x in registers, at the shapes where its split of K and N changes."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from cross_dsl_kernels_b200 import quantization as qz
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("k,n,group", [
+    (128, 8, 32),         # half a slice, half a column group
+    (384, 40, 64),        # a last slice of 128 k
+    (1280, 9008, 128),    # five slices: three column sets per CTA, several passes each
+    (3968, 2376, 128),    # the widest single CTA (15.5 slices)
+    (4352, 4096, 256),    # 17 slices: the first shape that a cluster shares, an uneven second rank
+    (11008, 1000, 128),   # 43 slices over three ranks
+    (14336, 528, 64),     # few column groups: more ranks than K alone asks for
+    (16384, 30000, 128),  # many passes per cluster
+    (32768, 24, 128),     # the longest K of the path
+    (32896, 24, 128),     # and the first one past it
+])
+@pytest.mark.parametrize("m", [1, 8, 9, 16])
+def test_w4a16_slices_ranks_and_sets(m, k, n, group):
+    """Codes, scales and x are small integers and powers of two: every sum is exact, whatever the order, so each of the
+    plans has to give the bits of a 64-bit product."""
+    from cross_dsl_kernels_b200.w4a16 import w4a16_linear
+    g = torch.Generator().manual_seed(k + n + m)
+    q = torch.randint(-1, 2, (n, k), generator=g, dtype=torch.int8)
+    packed = qz.pack_int4(q)
+    scales = torch.full((n, -(-k // group)), 0.5).half() * (1 + torch.randint(0, 2, (n, -(-k // group)), generator=g)).half()
+    x = (torch.randint(0, 16, (m, k), generator=g) == 0).half() * torch.randint(-1, 2, (m, k), generator=g).half()
+    bias = torch.randint(-4, 5, (n,), generator=g).half()
+    w = q.double() * scales.double().repeat_interleave(group, dim=1)[:, :k]
+    want = (x.double() @ w.t() + bias.double()).half()  # sums stay below 2^10 in halves: exact in FP16
+    for dependent in (False, True):
+        got = w4a16_linear(x.cuda(), packed.cuda(), scales.cuda(), bias.cuda(), group_size=group, dependent_launch=dependent)
+        assert torch.equal(got.cpu(), want)
