@@ -177,6 +177,9 @@ class DecodeLayerChain:
         self.k_cache = torch.full(shape, -999.0, dtype=torch.float16, device=self.device)
         self.v_cache = torch.full(shape, -999.0, dtype=torch.float16, device=self.device)
         self.arena = None
+        # a bound on the contexts from which the attention read splits the batch evenly adds its merge launch
+        merge = int(attention and _native.lib().xdk_paged_decode_attention_scratch_bytes(
+            c.tokens, hq, hkv, d, c.context, _native.XDK_F16) > 0)
         if world > 1 and exchange == "peer":
             from .peer import PeerArena
 
@@ -189,7 +192,7 @@ class DecodeLayerChain:
             self.q_peer = [self.arena.matrix(c.tokens, c.hidden, torch.float16) for _ in range(2)]
             self.up_peer = [self.arena.matrix(c.tokens, c.mlp if attention else 2 * c.mlp, torch.float16) for _ in range(2)]
             self.site_q, self.site_up = self.arena.new_site(), self.arena.new_site()
-            self.launches_per_layer = 9 if attention else 7  # the kernels + two flag barriers
+            self.launches_per_layer = 9 + merge if attention else 7  # the kernels + two flag barriers
         elif world > 1:
             self.q_gather = torch.empty(world, c.tokens, hq * d, dtype=torch.float16, device=self.device)
             self.up_gather = torch.empty(world, c.tokens, 2 * c.mlp // world, dtype=torch.float16, device=self.device)
@@ -197,7 +200,7 @@ class DecodeLayerChain:
             self.up_full = torch.empty(c.tokens, 2 * c.mlp, dtype=torch.float16, device=self.device)
             self.launches_per_layer = 7  # five kernels + two re-layout kernels (+ two NCCL all-gathers)
         else:
-            self.launches_per_layer = 7 if attention else 5
+            self.launches_per_layer = 7 + merge if attention else 5
 
     def host_weights(self, layer: int = 0) -> dict:
         """CPU copies of one layer's unsharded weights (single-rank chains only; for checkers)."""

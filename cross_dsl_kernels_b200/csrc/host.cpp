@@ -281,10 +281,15 @@ PyObject* attention(PyObject*, PyObject* const* arg, Py_ssize_t n) {
     Unlocked unlocked;
     c10::cuda::CUDAGuard guard(q.device());
     out = at::empty_like(q);
-    st = xdk_paged_decode_attention(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), pos.const_data_ptr<int64_t>(),
-                                    table.const_data_ptr<int64_t>(), seq.const_data_ptr<int64_t>(), out.data_ptr(), tokens, hq, hkv,
-                                    dim, table.size(1), page, hnd, static_cast<float>(scale), hint, code, launch_flags(dep),
-                                    stream_of(q));
+    const size_t need = xdk_paged_decode_attention_scratch_bytes(tokens, hq, hkv, dim, hint, code);
+    at::Tensor scratch;
+    if (need) scratch = at::empty({static_cast<int64_t>(need)}, q.options().dtype(at::kByte));
+    xdk_peer_out dst = {};
+    dst.ptr[0] = out.data_ptr(), dst.world = 1, dst.ld = hq * dim, dst.col0 = 0;
+    st = xdk_paged_decode_attention_ws(
+        q.data_ptr(), kc.data_ptr(), vc.data_ptr(), pos.const_data_ptr<int64_t>(), table.const_data_ptr<int64_t>(),
+        seq.const_data_ptr<int64_t>(), &dst, tokens, hq, hkv, dim, table.size(1), page, hnd, static_cast<float>(scale), hint, code,
+        need ? scratch.data_ptr() : nullptr, need, launch_flags(dep), stream_of(q));
   }
   return finish(st, "xdk_paged_decode_attention", THPVariable_Wrap(std::move(out)));
   END_HANDLE_TH_ERRORS

@@ -254,17 +254,22 @@ def paged_decode_attention(q, k_cache, v_cache, positions, page_table, sequence_
     scale = float(head_dim) ** -0.5 if scale is None else float(scale)
     _need(math.isfinite(scale), "scale must be finite")
     with torch.cuda.device(q.device):
-        tail = (tokens, q_heads, kv_heads, head_dim, page_table.shape[1], page_size, int(layout == "HND"), scale,
-                int(context_hint), _native.dtype_code(dtype), _flags(dependent_launch), _native.stream_ptr(q.device))
-        head = (q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), positions.data_ptr(), page_table.data_ptr(),
-                sequence_ids.data_ptr())
+        lib, code = _native.lib(), _native.dtype_code(dtype)
         if peer_out is None:
             out = torch.empty_like(q)
-            status = _native.lib().xdk_paged_decode_attention(*head, out.data_ptr(), *tail)
+            dst = _native.PeerOutStruct()
+            dst.ptr[0], dst.world, dst.ld, dst.col0 = out.data_ptr(), 1, q_heads * head_dim, 0
         else:
             _need(peer_out.ld >= peer_out.col0 + q_heads * head_dim, "peer_out is narrower than col0 + q_heads * head_dim")
-            out = None
-            status = _native.lib().xdk_paged_decode_attention_peer(*head, ctypes.byref(peer_out), *tail)
+            out, dst = None, peer_out
+        # partial results of (token, KV head) pairs that several CTAs share: a fresh block per call, as in decode_linear
+        need = lib.xdk_paged_decode_attention_scratch_bytes(tokens, q_heads, kv_heads, head_dim, int(context_hint), code)
+        scratch = torch.empty(need, device=q.device, dtype=torch.uint8) if need else None
+        status = lib.xdk_paged_decode_attention_ws(
+            q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), positions.data_ptr(), page_table.data_ptr(),
+            sequence_ids.data_ptr(), ctypes.byref(dst), tokens, q_heads, kv_heads, head_dim, page_table.shape[1], page_size,
+            int(layout == "HND"), scale, int(context_hint), code, scratch.data_ptr() if need else None, need,
+            _flags(dependent_launch), _native.stream_ptr(q.device))
     _native.check(status, "xdk_paged_decode_attention")
     return out
 

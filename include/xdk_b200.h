@@ -278,6 +278,21 @@ XDK_API int xdk_paged_decode_attention_peer(const void* q, const void* k_cache, 
                                     int64_t tokens, int64_t q_heads, int64_t kv_heads, int64_t head_dim,
                                     int64_t max_pages_per_seq, int64_t page_size, int cache_is_hnd, float scale,
                                     int64_t context_hint, int dtype, unsigned flags, void* stream);
+/*
+ * The attention read with device scratch from the caller (16-byte aligned, xdk_paged_decode_attention_scratch_bytes bytes
+ * or more, its content undefined before and after; not shared by calls that may overlap on the GPU): the tiles of all
+ * tokens' contexts are dealt evenly to the CTAs, whatever the mix of context lengths, and a second launch merges, in a
+ * fixed order, what several CTAs hold of a (token, KV head).  Without scratch (NULL, or fewer bytes; the size function
+ * returns 0 for what it does not take, short contexts among it) it is the call above.
+ */
+XDK_API size_t xdk_paged_decode_attention_scratch_bytes(int64_t tokens, int64_t q_heads, int64_t kv_heads, int64_t head_dim,
+                                                int64_t context_hint, int dtype);
+XDK_API int xdk_paged_decode_attention_ws(const void* q, const void* k_cache, const void* v_cache, const int64_t* positions,
+                                  const int64_t* page_table, const int64_t* sequence_ids, const xdk_peer_out* out_dst,
+                                  int64_t tokens, int64_t q_heads, int64_t kv_heads, int64_t head_dim,
+                                  int64_t max_pages_per_seq, int64_t page_size, int cache_is_hnd, float scale,
+                                  int64_t context_hint, int dtype, void* scratch, size_t scratch_bytes, unsigned flags,
+                                  void* stream);
 XDK_API int xdk_swiglu_peer(const void* upgate, const xdk_peer_out* out_dst, int64_t rows, int64_t width, int64_t in_ld,
                     int dtype, unsigned flags, void* stream);
 

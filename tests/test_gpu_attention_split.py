@@ -1,0 +1,62 @@
+"""Attention over contexts of every mix: the even split over the CTAs, with and without scratch."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from conftest import rel_l2
+from oracle import attention as oracle_attention
+
+pytestmark = pytest.mark.gpu
+
+
+def _paged(tokens, q_heads, kv_heads, dim, page, positions, dtype, seed):
+    g = torch.Generator().manual_seed(seed)
+    per_seq = max(positions) // page + 1
+    table = torch.randperm(tokens * per_seq, generator=g).reshape(tokens, per_seq)
+    shape = (tokens * per_seq, page, kv_heads, dim)
+    return (torch.randn(tokens, q_heads, dim, generator=g).to(dtype), torch.randn(shape, generator=g).to(dtype),
+            torch.randn(shape, generator=g).to(dtype), torch.tensor(positions), table, torch.arange(tokens))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("heads,dim,page,positions", [
+    ((32, 8), 128, 16, [8191]),                                  # one long context over every CTA
+    ((8, 1), 64, 16, [0, 3000, 63, 64, 1, 127, 128, 2047]),      # items inside one CTA, across two, across many
+    ((4, 4), 256, 5, [700, 0, 0, 0, 15, 16, 31]),                # odd pages, whole tiles and single positions
+    ((2, 2), 64, 16, [0] * 3),                                   # fewer tiles than CTAs
+    ((4, 2), 64, 7, [i % 90 for i in range(300)]),               # more tokens than a block has threads
+])
+def test_attention_even_split(dtype, heads, dim, page, positions):
+    """Contexts of every mix, dealt evenly to the CTAs: against the FP32 restatement, for each bound the caller may name
+    (the grid follows it), and the same bits from the split over heads and clusters that runs without scratch."""
+    from cross_dsl_kernels_b200 import _native
+    from cross_dsl_kernels_b200.ops import paged_decode_attention
+    q, kc, vc, pos, table, seq = _paged(len(positions), *heads, dim, page, positions, dtype, seed=dim + len(positions))
+    want = oracle_attention.paged_decode_attention(q, kc, vc, pos, table, seq, page_size=page)
+    dev = [t.cuda() for t in (q, kc, vc, pos, table, seq)]
+    rel = 1e-5 if dtype == torch.float32 else 1e-3  # of the existing attention tests
+    for hint in (0, 1, 100, max(positions) + 1, 100000):
+        got = paged_decode_attention(*dev, page_size=page, context_hint=hint)
+        assert rel_l2(got.cpu(), want) <= rel
+        assert torch.equal(got, paged_decode_attention(*dev, page_size=page, context_hint=hint)), "deterministic"
+    bare = torch.empty_like(dev[0])
+    status = _native.lib().xdk_paged_decode_attention(
+        *(t.data_ptr() for t in dev), bare.data_ptr(), len(positions), *heads, dim, table.shape[1], page, 0, dim ** -0.5, 0,
+        _native.dtype_code(dtype), 0, _native.stream_ptr(bare.device))
+    _native.check(status, "attention without scratch")
+    assert rel_l2(bare.cpu(), want) <= rel
+
+
+def test_attention_not_a_number_and_empty_contexts_show():
+    """A NaN in one row of K reaches exactly the heads that read it, split or not; a position of -1 (nothing to attend to)
+    gives NaN, as 0 / 0 always did."""
+    from cross_dsl_kernels_b200.ops import paged_decode_attention
+    q, kc, vc, pos, table, seq = _paged(3, 8, 2, 128, 16, [4000, 5, 2000], torch.float16, seed=3)
+    page, off = int(table[0, 2500 // 16]), 2500 % 16
+    kc[page, off, 1] = float("nan")
+    pos[1] = -1
+    got = paged_decode_attention(*(t.cuda() for t in (q, kc, vc, pos, table, seq)), page_size=16).cpu()
+    assert torch.isnan(got[0, 4:]).all() and torch.isfinite(got[0, :4]).all()
+    assert torch.isnan(got[1]).all() and torch.isfinite(got[2]).all()
