@@ -994,12 +994,18 @@ w4a16_generic_kernel(W4Args a) {
 // memory in warp order.  A warp's work is a sequence of batches (a column pass x a round of up to four 128-k chunks
 // of its K share); the loads of the next batch are in flight while the current one is unpacked and multiplied, in
 // two register buffers, so the weight stream never waits for the tensor pipe nor the pipe for the stream.
+//
+// Two shapes of it: batches of four chunks and two CTAs per SM (127 registers), or of two chunks and three (80), for more
+// column groups than two CTAs per SM take in one pass each, while x is small enough to leave the third CTA room and the L1
+// cache its scales.
+template <int CHUNKS>
 struct MmaBatch {
-  U4 wv[4][2];      // [chunk][column n, column n + 8]: 32 codes each
-  __half2 sc[4][2]; // their scale, in both halves
+  U4 wv[CHUNKS][2];       // [chunk][column n, column n + 8]: 32 codes each
+  __half2 sc[CHUNKS][2];  // their scale, in both halves
 };
 
-__global__ void __launch_bounds__(kThreads, 2)
+template <int CHUNKS, int CTAS>
+__global__ void __launch_bounds__(kThreads, CTAS)
 w4a16_mma_kernel(W4Args a, int col_groups) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int pitch = a.k * 2 + 16;                          // bytes per x row: the pad puts the 8 rows on different banks
@@ -1010,7 +1016,7 @@ w4a16_mma_kernel(W4Args a, int col_groups) {
   const int row_bytes = a.k / 2;
   const int k_warp = a.k / kWarps;          // this warp's share of K, a multiple of 128
   const int chunks = k_warp / 128;          // 128 k per chunk: 32 per lane of a quad
-  constexpr int kBatchChunks = 4;
+  constexpr int kBatchChunks = CHUNKS;
   const int rounds = (chunks + kBatchChunks - 1) / kBatchChunks;
   const int k0 = warp * k_warp + q * 32;    // first k of this lane's vectors
   // the groups of 16 columns are dealt evenly to the CTAs of the grid (all resident at once: no second wave)
@@ -1021,7 +1027,7 @@ w4a16_mma_kernel(W4Args a, int col_groups) {
   const int scale_shift = 31 - __clz(a.group);  // group sizes are powers of two
   // Columns past N (the last pass of the last CTA when N % 16 != 0) read the last column instead and chunks past the
   // warp's share are not loaded at all: what they would feed is never stored, respectively never computed.
-  auto fetch = [&](MmaBatch& b, int col_base, int chunk0) {
+  auto fetch = [&](MmaBatch<CHUNKS>& b, int col_base, int chunk0) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int col = min(col_base + h * 8 + n, a.n - 1), k = k0 + chunk0 * 128;
@@ -1035,7 +1041,7 @@ w4a16_mma_kernel(W4Args a, int col_groups) {
         }
     }
   };
-  MmaBatch buf0, buf1;
+  MmaBatch<CHUNKS> buf0, buf1;
   pdl_launch_dependents();
   fetch(buf0, cta_col0, 0);  // the first batch's weights go out before x is staged
   pdl_wait();                // x may be the preceding kernel's output; the weights are not
@@ -1059,7 +1065,7 @@ w4a16_mma_kernel(W4Args a, int col_groups) {
   // (column n, rows 2 q + {0, 1} of x), (column n + 8, the same rows)
   float acc0[4], acc1[4];
   int pass = 0, round = 0;  // of the batch being computed
-  auto step = [&](MmaBatch& cur, MmaBatch& nxt) -> bool {
+  auto step = [&](MmaBatch<CHUNKS>& cur, MmaBatch<CHUNKS>& nxt) -> bool {
     int np = pass, nr = round + 1;
     if (nr == rounds) nr = 0, ++np;
     const bool has_next = np < my_passes;
@@ -1120,20 +1126,21 @@ w4a16_mma_kernel(W4Args a, int col_groups) {
   }
 }
 
+template <int CHUNKS, int CTAS>
 int launch_mma(W4Args a, bool dependent, cudaStream_t stream) {
   const size_t xbytes = (static_cast<size_t>(a.m) * (a.k * 2 + 16) + 127) & ~static_cast<size_t>(127);
   const size_t smem = xbytes + 2 * static_cast<size_t>(kWarps) * 32 * 4 * sizeof(float);
-  cudaError_t err = cudaFuncSetAttribute(w4a16_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  cudaError_t err = cudaFuncSetAttribute(w4a16_mma_kernel<CHUNKS, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (err != cudaSuccess) return note_launch(err);
   // one wave: as many CTAs as the device holds at once (two per SM unless x takes more than half the shared memory);
   // a grid of a few CTAs more than that ran as two waves and took twice the time
   int resident = 0;
-  err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, w4a16_mma_kernel, kThreads, smem);
+  err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, w4a16_mma_kernel<CHUNKS, CTAS>, kThreads, smem);
   if (err != cudaSuccess) return note_launch(err);
   if (resident < 1) return XDK_ERR_LIMIT;
   const int groups = (a.n + 15) / 16;
   const int ctas = groups < resident * sm_count() ? groups : resident * sm_count();
-  return launch_opts(w4a16_mma_kernel, dim3(ctas), dim3(kThreads), smem, stream, 1u, dependent, a, groups);
+  return launch_opts(w4a16_mma_kernel<CHUNKS, CTAS>, dim3(ctas), dim3(kThreads), smem, stream, 1u, dependent, a, groups);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1529,7 +1536,15 @@ extern "C" int xdk_w4a16_peer(const void* x, const uint8_t* packed, const void* 
   static const int umma_env = getenv("XDK_W4A16_UMMA") ? (getenv("XDK_W4A16_UMMA")[0] == '1' ? 1 : 0) : -1;
   const size_t x_bytes = static_cast<size_t>(m) * (static_cast<size_t>(k) * 2 + 16);
   if (mma_env && plain && vec_ok && k % 1024 == 0 && (m <= 2 ? x_bytes <= 160 * 1024 : m <= 8 && x_bytes <= 104 * 1024))
-    return launch_mma(a, dependent, s);
+  {
+    // Three CTAs per SM where that saves a pass over the column groups, or K is short (us with two / three, M = 1: K = 4096,
+    // N = 6144 9.3 / 7.7, N = 20480 17.6 / 16.0, N = 28672 23.3 / 22.8, N = 8192 -- two passes either way -- 9.7 / 10.6; K = 2048,
+    // N = 8192 6.6 / 6.3, N = 28672 16.1 / 13.8; M = 4 alike).  A larger x leaves the L1 cache too little for the scales.
+    const int64_t groups = (n + 15) / 16, two = 2LL * sm_count(), three = 3LL * sm_count();
+    if (x_bytes <= 40 * 1024 && k <= 4096 && groups > two && (k <= 2048 || (groups + three - 1) / three < (groups + two - 1) / two))
+      return launch_mma<2, 3>(a, dependent, s);
+    return launch_mma<4, 2>(a, dependent, s);
+  }
   const bool umma_ok = vec_ok && k % 256 == 0 && group_size >= 64 && a.groups <= 256 && a.groups % 8 == 0 && aligned16(scales);
   const int64_t units = ((n + 31) / 32 + sm_count() - 1) / sm_count();  // 32-column units of the tcgen05 kernel's busiest CTA
   const bool whole = units % 4 == 0 || units == 3 || (units == 2 && k < 8192) || (units > 4 && k > 4096);

@@ -1,4 +1,5 @@
-"""The W4A16 kernel that keeps x in registers, at the shapes where its split of K and N changes."""
+"""The W4A16 kernel that keeps x in registers, at the shapes where its split of K and N changes, and the two shapes of the
+direct-load kernel."""
 
 from __future__ import annotations
 
@@ -19,6 +20,8 @@ pytestmark = pytest.mark.gpu
     (11008, 1000, 128),   # 43 slices over three ranks
     (14336, 528, 64),     # few column groups: more ranks than K alone asks for
     (16384, 30000, 128),  # many passes per cluster
+    (3072, 4800, 128),    # few rows: three CTAs per SM save the direct-load kernel a pass; three chunks in batches of two
+    (2048, 28680, 64),    # and several passes of it, a ragged last one
     (32768, 24, 128),     # the longest K of the path
     (32896, 24, 128),     # and the first one past it
 ])
