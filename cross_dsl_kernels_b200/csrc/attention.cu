@@ -52,13 +52,15 @@ struct AttnArgs {
   float* scratch;  // even split of the batch's tiles over the grid, partial results here; nullptr: grid = (splits, heads, tokens)
 };
 
-// 16 bytes at byte offset `at` of a cache row, or zeros and no access for a dead position (row < 0).  (Dead positions used to
-// read row 0 of the cache: with contexts of every length that was megabytes from one line, and its L2 slice set the time --
-// 64 contexts of 1 .. 2048 took longer than 64 of 2048.)
+// 16 bytes, or zeros and no access (bytes = 0) for a dead position.  (Dead positions used to read row 0 of the cache: with
+// contexts of every length that was megabytes from one line, and its L2 slice set the time -- 64 contexts of 1 .. 2048 took
+// longer than 64 of 2048.)
+__device__ __forceinline__ void cp_async16_or_zero(void* dst_smem, const unsigned char* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst_smem)), "l"(src), "r"(bytes) : "memory");
+}
 template <typename T>
-__device__ __forceinline__ void cp_async16_row(void* dst_smem, const T* cache, int64_t row, int at) {
-  const unsigned char* src = reinterpret_cast<const unsigned char*>(cache + (row < 0 ? 0 : row)) + at;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst_smem)), "l"(src), "r"(row < 0 ? 0 : 16) : "memory");
+__device__ __forceinline__ void cp_async16_row(void* dst_smem, const T* cache, int64_t row, int at) {  // row < 0: dead
+  cp_async16_or_zero(dst_smem, reinterpret_cast<const unsigned char*>(cache + (row < 0 ? 0 : row)) + at, row < 0 ? 0 : 16);
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
@@ -82,8 +84,9 @@ constexpr int kMaxTokensSplit = 16384;  // every CTA adds up the tiles of all to
 // Shorter contexts stay on the grid of splits: finding the share and the second launch cost about 4 us, which the even split
 // only earns back on uneven or long ones.  us, contexts of every length up to the bound / all at the bound, even against
 // splits: 16 tokens x 8 heads x 128, bound 512 13.8 / 13.3 against 12.3 / 14.9, 1024 15.9 / 19.4 against 15.9 / 18.1, 2048
-// 20.0 / 33.2 against 24.1 / 32.9, 8192 58 / 97 against 82 / 98 at the start; 64 tokens, 2048 61 / 98 against 103 / 122 at the
-// start; one token, 8192 13.9 / 16.8 against 14.9 / 24.8; FP32, 64 tokens x 4 heads, 2048 63 / 102 against 123 / 131.
+// 20.0 / 33.2 against 24.1 / 32.9; one token, 8192 13.9 / 16.8 against 14.9 / 24.8; FP32, 64 tokens x 4 heads, 2048 63 / 102 against 123 / 131.
+// Against the kernel before the even split, whose dead positions were read: 16 tokens, 8192 56 / 95 from 82 / 98; 64 tokens,
+// 2048 58 / 96 from 103 / 122.
 constexpr int kMinEvenContext = 1536;
 
 template <int G, int D>
@@ -629,7 +632,7 @@ paged_decode_attention_tc_kernel(const T* __restrict__ q, const T* __restrict__ 
   extern __shared__ __align__(16) unsigned char attn_smem[];
   unsigned char* ktile = attn_smem + warp_of(threadIdx.x) * Tile::kStage;
   unsigned char* vtile = ktile + TP * kPitch;
-  __shared__ int64_t rows[kAttnWarps][TP];
+  __shared__ uintptr_t rows[kAttnWarps][TP];  // addresses of the tile's K rows
   __shared__ float part_m[kAttnWarps][G], part_l[kAttnWarps][G];
   __shared__ float cta_m[G], cta_l[G];
   __shared__ int64_t batch_tiles;
@@ -657,6 +660,8 @@ paged_decode_attention_tc_kernel(const T* __restrict__ q, const T* __restrict__ 
     n_tiles = static_cast<int>(static_cast<int64_t>(cur.tiles) * (split + 1) / splits) - cur.tile;
   }
 
+  // V rows lie where the K rows lie, this many bytes on
+  const int64_t v_from_k = static_cast<int64_t>(reinterpret_cast<uintptr_t>(v_cache) - reinterpret_cast<uintptr_t>(k_cache));
   RowAt at;  // this lane's row of the tile
   auto look_up = [&]() { at.find(a, cur, static_cast<int64_t>(cur.tile) * Tile::kUnit + warp * TP + lane); };
   if (n_tiles > 0) look_up();
@@ -700,21 +705,20 @@ paged_decode_attention_tc_kernel(const T* __restrict__ q, const T* __restrict__ 
   if (n_tiles == 0) begin_segment(cur.token, cur.kvh);  // a split without tiles (more splits than tiles) contributes nothing
 
   for (int u = 0; u < n_tiles; ++u) {
-    rows[warp][lane] = at.offset(a, cur.kvh, D);
+    rows[warp][lane] = reinterpret_cast<uintptr_t>(k_cache) + (at.page < 0 ? 0 : at.offset(a, cur.kvh, D) * static_cast<int64_t>(sizeof(T)));
     __syncwarp();
-    // K and V rows of the tile, 16 bytes per lane and instruction: one trip to HBM
-#pragma unroll
-    for (int i = 0; i < PIECES; ++i) {
-      const int c = i * 32 + lane, r = c / PIECES, p = c - r * PIECES;
-      cp_async16_row(ktile + r * kPitch + p * 16, k_cache, rows[warp][r], p * 16);
-    }
-#pragma unroll
-    for (int i = 0; i < PIECES; ++i) {
-      const int c = i * 32 + lane, r = c / PIECES, p = c - r * PIECES;
-      cp_async16_row(vtile + r * kPitch + p * 16, v_cache, rows[warp][r], p * 16);
-    }
     const int64_t rest = cur.ctx - static_cast<int64_t>(cur.tile) * Tile::kUnit - warp * TP;
     const int live_end = rest < TP ? static_cast<int>(rest > 0 ? rest : 0) : TP;  // of this warp's positions
+    // K and V rows of the tile, 16 bytes per lane and instruction: one trip to HBM.  Dead positions, the last ones of the
+    // tile, are zero-filled and not read.
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {
+      const int c = i * 32 + lane, r = c / PIECES, p = c - r * PIECES;
+      const unsigned char* src = reinterpret_cast<const unsigned char*>(rows[warp][r]) + p * 16;
+      const int bytes = r < live_end ? 16 : 0;
+      cp_async16_or_zero(ktile + r * kPitch + p * 16, src, bytes);
+      cp_async16_or_zero(vtile + r * kPitch + p * 16, src + v_from_k, bytes);
+    }
     const int token = cur.token, kvh = cur.kvh, tiles_left = cur.tiles - 1 - cur.tile;
     if (fresh) {
       begin_segment(token, kvh);

@@ -1345,7 +1345,7 @@ w4a16_rx_kernel(W4Args a, RxPlan plan, const __grid_constant__ CUtensorMap wmap)
       }
     }
     __syncwarp();  // every lane has read the slot
-    if (lane == 0 && pass + depth < passes) issue(slot.slot, pass + depth);
+    if (lane == 0 && ok && pass + depth < passes) issue(slot.slot, pass + depth);
     slot.advance(depth);
     if (ok) ok = mbar_wait(part_empty + pb.slot, pb.parity ^ 1u);  // a fresh barrier passes: nothing is parked yet
     float4* mine = part + (pb.slot * plan.cta_slices + ws) * MR * 32 + lane;
