@@ -41,3 +41,20 @@ def test_w4a16_slices_ranks_and_sets(m, k, n, group):
     for dependent in (False, True):
         got = w4a16_linear(x.cuda(), packed.cuda(), scales.cuda(), bias.cuda(), group_size=group, dependent_launch=dependent)
         assert torch.equal(got.cpu(), want)
+
+
+@pytest.mark.parametrize("m,k", [(3, 384), (8, 1152), (9, 128), (16, 5504)])
+def test_w4a16_large_scales_on_a_last_half_slice(m, k):
+    """K % 256 = 128 leaves half of the last slice past K, where the copy fills the codes with zeros; a zero code stands for
+    -8, and with a scale of 8192 or more -8 * scale is an infinity in FP16.  The quantizer gives such scales."""
+    from cross_dsl_kernels_b200.w4a16 import w4a16_linear
+    w = torch.zeros(24, k)
+    w[:, ::37] = 60000.0
+    packed, scales = qz.quantize_int4(w.half(), group_size=128)
+    assert scales.max() >= 8192
+    x = torch.zeros(m, k).half()
+    x[:, ::37] = 2.0 ** -12
+    got = w4a16_linear(x.cuda(), packed.cuda(), scales.cuda(), group_size=128).cpu()
+    codes = qz.unpack_int4(packed, k).double()
+    want = x.double() @ (codes * scales.double().repeat_interleave(128, dim=1)[:, :k]).half().double().t()
+    assert torch.equal(got, want.half())
