@@ -88,6 +88,9 @@ constexpr int kMaxTokensSplit = 16384;  // every CTA adds up the tiles of all to
 // Against the kernel before the even split, whose dead positions were read: 16 tokens, 8192 56 / 95 from 82 / 98; 64 tokens,
 // 2048 58 / 96 from 103 / 122.
 constexpr int kMinEvenContext = 1536;
+// A larger bound on the contexts says no more than this one: it is far beyond any cache, and keeps tokens * heads * tiles, and the
+// roundings up, inside 64 bits.
+constexpr int64_t kMaxContextHint = 1LL << 38;
 
 template <int G, int D>
 struct Partials {  // scratch of a grid of `ctas`
@@ -850,7 +853,8 @@ paged_decode_attention_tc_kernel(const T* __restrict__ q, const T* __restrict__ 
 // CTAs of a launch that splits the batch evenly (0: the batch stays on the grid of splits): what the SMs hold at once, and
 // no more than leaves every CTA as many tiles as the busiest would have anyway, by the bound on the contexts.
 inline int even_grid(int64_t tokens, int64_t kv_heads, int64_t dim, int64_t hint, int elem, int g) {
-  if (tokens > kMaxTokensSplit || (hint > 0 && hint < kMinEvenContext)) return 0;
+  if (tokens > kMaxTokensSplit || kv_heads > 65535 || (hint > 0 && hint < kMinEvenContext)) return 0;
+  if (hint > kMaxContextHint) hint = kMaxContextHint;
   const bool stage_v = kAttnWarps * 32 * (2 * dim * elem + 16) <= 72 * 1024;  // StageV of the FP32 kernel
   int64_t smem = elem == 4 ? kAttnWarps * 32 * ((stage_v ? 2 : 1) * dim * elem + 16) : kAttnWarps * 64 * (dim * 2 + 16);
   smem += elem == 4 ? g * dim * 4 + kAttnWarps * 32 * (g * 4 + 8) + 3840 : 4608;  // static and reserved
@@ -991,6 +995,7 @@ extern "C" int xdk_paged_decode_attention_ws(const void* q, const void* k_cache,
   if (tokens < 1 || q_heads < 1 || kv_heads < 1 || head_dim < 1 || max_pages_per_seq < 1 || page_size < 1) return XDK_ERR_ARG;
   if (q_heads % kv_heads != 0 || !(scale == scale)) return XDK_ERR_ARG;
   if (tokens > 65535 || kv_heads > 65535) return XDK_ERR_LIMIT;
+  if (context_hint > kMaxContextHint) context_hint = kMaxContextHint;
   if (!aligned16(q) || !aligned16(k_cache) || !aligned16(v_cache)) return XDK_ERR_ARG;
   if (int st = require_sm100()) return st;
   AttnArgs a;
