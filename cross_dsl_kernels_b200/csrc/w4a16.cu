@@ -1228,15 +1228,17 @@ w4a16_rx_kernel(W4Args a, RxPlan plan, const __grid_constant__ CUtensorMap wmap)
   const int scale_shift = 31 - __clz(a.group);
   int scale_idx[2];
 #pragma unroll
-  for (int c = 0; c < 2; ++c) scale_idx[c] = k0 + c * 128 < a.k ? (k0 + c * 128) >> scale_shift : -1;
+  for (int c = 0; c < 2; ++c) scale_idx[c] = min((k0 + c * 128) >> scale_shift, a.groups - 1);
+  // A second chunk past K (the first one never is) has codes of zero, which stand for -8: its scale counts as zero, any above
+  // 8188 would make infinities of them.
+  const uint32_t second_live = k0 + 128 < a.k ? 0xffffffffu : 0u;
   __half scale_next[2][2];
   auto fetch_scales = [&](int pass) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {  // past N: any column, its sums are not stored
       const __half* at = a.scales + static_cast<size_t>(min((g0 + pass) * 16 + h * 8 + col_lo, a.n - 1)) * a.groups;
 #pragma unroll
-      for (int c = 0; c < 2; ++c)  // a chunk past K has codes of zero, which stand for -8: any scale above 8188 would make infinities
-        scale_next[c][h] = scale_idx[c] >= 0 ? __ldg(at + scale_idx[c]) : __ushort_as_half(0);
+      for (int c = 0; c < 2; ++c) scale_next[c][h] = __ldg(at + scale_idx[c]);
     }
   };
   fetch_scales(0);
@@ -1318,7 +1320,11 @@ w4a16_rx_kernel(W4Args a, RxPlan plan, const __grid_constant__ CUtensorMap wmap)
 #pragma unroll
     for (int c = 0; c < 2; ++c)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) sc[c][h] = __half2half2(scale_next[c][h]);
+      for (int h = 0; h < 2; ++h) {
+        const __half2 both = __half2half2(scale_next[c][h]);
+        const uint32_t bits = *reinterpret_cast<const uint32_t*>(&both) & (c ? second_live : 0xffffffffu);
+        sc[c][h] = *reinterpret_cast<const __half2*>(&bits);
+      }
     if (pass + 1 < passes) fetch_scales(pass + 1);
     if (ok) ok = mbar_wait(full + slot.slot, slot.parity);
     float acc[MR][4];
