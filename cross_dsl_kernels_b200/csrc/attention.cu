@@ -296,7 +296,7 @@ struct RowAt {
     if (a.narrow) logical = static_cast<uint32_t>(j) / static_cast<uint32_t>(a.page_size);
     else logical = j / a.page_size;
     off = static_cast<int>(j - logical * a.page_size);
-    page = __ldg(c.table + logical);
+    page = c.table[logical];
   }
   __device__ __forceinline__ int64_t offset(const AttnArgs& a, int kvh, int dim) const {
     if (page < 0) return -1;
@@ -311,7 +311,7 @@ struct StageV {  // whether a warp's V rows are staged in shared memory beside i
 
 template <typename T, int G, int D>
 __global__ void __launch_bounds__(kAttnThreads)
-paged_decode_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
+paged_decode_attention_kernel(const T* q, const T* k_cache, const T* v_cache,
                               const __grid_constant__ PeerOut out, const __grid_constant__ AttnArgs a, int splits) {
   constexpr int E = 16 / sizeof(T);   // elements per 16-byte piece
   constexpr int PIECES = D / E;       // pieces per row
@@ -478,12 +478,12 @@ paged_decode_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_c
       for (int u = 0; u < 4; ++u) {
         const T* vp = v_cache + rows[warp][min(j0 + u, n_live - 1)] + lane * DPL;
         if constexpr (DPL * sizeof(T) == 8) {
-          const uint2 raw = __ldg(reinterpret_cast<const uint2*>(vp));
+          const uint2 raw = *reinterpret_cast<const uint2*>(vp);
           const T* ve = reinterpret_cast<const T*>(&raw);
 #pragma unroll
           for (int e = 0; e < DPL; ++e) vf[u][e] = Elem<T>::to_f32(ve[e]);
         } else if constexpr (DPL * sizeof(T) == 16) {
-          const U4 raw = ld_stream16(vp);
+          const U4 raw = ld_ordered_stream16(vp);
           const T* ve = reinterpret_cast<const T*>(&raw);
 #pragma unroll
           for (int e = 0; e < DPL; ++e) vf[u][e] = Elem<T>::to_f32(ve[e]);
@@ -625,7 +625,7 @@ struct TcTile {
 
 template <typename T, int G, int D>
 __global__ void __launch_bounds__(kAttnThreads, D <= 128 ? 3 : 1)
-paged_decode_attention_tc_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
+paged_decode_attention_tc_kernel(const T* q, const T* k_cache, const T* v_cache,
                                  const __grid_constant__ PeerOut out, const __grid_constant__ AttnArgs a, int splits) {
   static_assert(sizeof(T) == 2 && G <= 8 && D % 32 == 0, "16-bit caches, at most eight heads per group");
   using Tile = TcTile<D>;

@@ -135,11 +135,26 @@ __device__ __forceinline__ U4 ld_cached16(const void* p) {
   const uint4 t = __ldg(reinterpret_cast<const uint4*>(p));
   return U4{t.x, t.y, t.z, t.w};
 }
-// 128-bit load of what the preceding kernel wrote.  Volatile, so that it stays behind pdl_wait(): a load through the
-// read-only path (ld_cached16) counts as invariant and the compiler may move it in front of the wait.
+// Loads of what the preceding kernel may have written: activations, caches, index tensors.  A load through the read-only path
+// (ld_cached16, ld_stream16, __ldg, or a plain one through a const __restrict__ pointer) counts as invariant, and the compiler
+// may move it in front of pdl_wait(); these stay behind it, as does a plain load through a pointer without __restrict__.
 __device__ __forceinline__ U4 ld_ordered16(const void* p) {
   U4 v;
   asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ U4 ld_ordered16_if(const void* p, bool live) {  // zeros and no access where not live; no branch
+  U4 v;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+      "@q ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}"
+      : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w) : "l"(p), "r"(static_cast<unsigned>(live)) : "memory");
+  return v;
+}
+__device__ __forceinline__ U4 ld_ordered_stream16(const void* p) {  // each byte is used once: not kept in L1
+  U4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ float4 ld_stream_f4(const float* p) {

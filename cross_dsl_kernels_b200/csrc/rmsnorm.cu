@@ -38,7 +38,7 @@ __device__ __forceinline__ float inv_rms(float sum_sq, float hidden_f, float eps
 // Row-resident vector kernel: thread t holds vectors t, t+THREADS, ... (VPT of them) of the row.
 template <typename T, int THREADS, int VPT>
 __global__ void __launch_bounds__(THREADS)
-rmsnorm_row_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T* __restrict__ weight,
+rmsnorm_row_kernel(const T* x, const T* residual, const T* __restrict__ weight,
                    T* __restrict__ y, T* __restrict__ residual_out, int nvec, float hidden_f, float eps) {
   constexpr int E = Elem<T>::kPerVec;
   __shared__ float scratch[THREADS / 32 + 1];
@@ -67,8 +67,8 @@ rmsnorm_row_kernel(const T* __restrict__ x, const T* __restrict__ residual, cons
   for (int i = 0; i < VPT; ++i) {
     const int v = threadIdx.x + i * THREADS;
     if (v < nvec) {
-      xin[i] = ld_stream16(xv + v);
-      rin[i] = ld_stream16(rv + v);
+      xin[i] = ld_ordered_stream16(xv + v);
+      rin[i] = ld_ordered_stream16(rv + v);
     }
   }
   float r[VPT][E];
@@ -107,7 +107,7 @@ rmsnorm_row_kernel(const T* __restrict__ x, const T* __restrict__ residual, cons
 // then) and recomputes the FP32 sum, it never reads back the rounded residual_out.
 template <typename T>
 __global__ void __launch_bounds__(256)
-rmsnorm_generic_kernel(const T* __restrict__ x, const T* __restrict__ residual, const T* __restrict__ weight,
+rmsnorm_generic_kernel(const T* x, const T* residual, const T* __restrict__ weight,
                        T* __restrict__ y, T* __restrict__ residual_out, int64_t hidden, float hidden_f,
                        float eps) {
   __shared__ float scratch[256 / 32 + 1];

@@ -23,7 +23,7 @@ template <typename T, int W> struct Chunk {
     if constexpr (W == 1) {
       f[0] = Elem<T>::to_f32(*p);
     } else {
-      unpack16<T>(ld_stream16(p), f);
+      unpack16<T>(ld_ordered_stream16(p), f);
     }
   }
   __device__ __forceinline__ void store(T* p) const {
@@ -53,10 +53,10 @@ __device__ __forceinline__ int64_t cache_row(const RopeShape& s, int64_t page, i
 
 template <typename T, int W, bool INTERLEAVED>
 __global__ void __launch_bounds__(128)
-rope_append_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
+rope_append_kernel(const T* q, const T* k, const T* v,
                    const float* __restrict__ cos, const float* __restrict__ sin,
-                   const int64_t* __restrict__ positions, const int64_t* __restrict__ page_table,
-                   const int64_t* __restrict__ sequence_ids, T* __restrict__ q_out, T* __restrict__ k_cache,
+                   const int64_t* positions, const int64_t* page_table,
+                   const int64_t* sequence_ids, T* __restrict__ q_out, T* __restrict__ k_cache,
                    T* __restrict__ v_cache, RopeShape s, int units_rot_head, int units_token) {
   pdl_launch_dependents();
   pdl_wait();  // q, k, v may be the preceding kernel's output; the caches may still be read by it
@@ -104,14 +104,14 @@ rope_append_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __
   if (second >= 0) b.load(src + src_row + static_cast<int64_t>(second) * W);
 
   // ---- dependent index chain
-  const int64_t pos = __ldg(positions + token);
+  const int64_t pos = positions[token];
   int64_t dst_row = static_cast<int64_t>(token) * s.qout.ld + s.qout.col0 + static_cast<int64_t>(head) * s.head_dim;
   T* dst = q_out;
   if (kind != 0) {
-    const int64_t seq = __ldg(sequence_ids + token);
+    const int64_t seq = sequence_ids[token];
     const int64_t logical = pos / s.page_size;
     const int64_t off = pos - logical * s.page_size;
-    const int64_t page = __ldg(page_table + seq * s.max_pages + logical);
+    const int64_t page = page_table[seq * s.max_pages + logical];
     dst_row = cache_row(s, page, off, head);
     dst = kind == 1 ? k_cache : v_cache;
   }
@@ -172,10 +172,10 @@ int launch_rope(const void* q, const void* k, const void* v, const float* cos, c
 // Scalar interleaved path: one thread per (head, pair) or per copied element.
 template <typename T>
 __global__ void __launch_bounds__(128)
-rope_append_scalar_interleaved_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
+rope_append_scalar_interleaved_kernel(const T* q, const T* k, const T* v,
                                       const float* __restrict__ cos, const float* __restrict__ sin,
-                                      const int64_t* __restrict__ positions, const int64_t* __restrict__ page_table,
-                                      const int64_t* __restrict__ sequence_ids, T* __restrict__ q_out,
+                                      const int64_t* positions, const int64_t* page_table,
+                                      const int64_t* sequence_ids, T* __restrict__ q_out,
                                       T* __restrict__ k_cache, T* __restrict__ v_cache, RopeShape s,
                                       int units_rot_head, int units_token) {
   pdl_launch_dependents();
@@ -208,14 +208,14 @@ rope_append_scalar_interleaved_kernel(const T* __restrict__ q, const T* __restri
   const int64_t src_row = static_cast<int64_t>(token) * stride + static_cast<int64_t>(head) * s.head_dim;
   float lo = Elem<T>::to_f32(src[src_row + d0]);
   float hi = d1 >= 0 ? Elem<T>::to_f32(src[src_row + d1]) : 0.0f;
-  const int64_t pos = __ldg(positions + token);
+  const int64_t pos = positions[token];
   int64_t dst_row = static_cast<int64_t>(token) * s.qout.ld + s.qout.col0 + static_cast<int64_t>(head) * s.head_dim;
   T* dst = q_out;
   if (kind != 0) {
-    const int64_t seq = __ldg(sequence_ids + token);
+    const int64_t seq = sequence_ids[token];
     const int64_t logical = pos / s.page_size;
     const int64_t off = pos - logical * s.page_size;
-    const int64_t page = __ldg(page_table + seq * s.max_pages + logical);
+    const int64_t page = page_table[seq * s.max_pages + logical];
     dst_row = cache_row(s, page, off, head);
     dst = kind == 1 ? k_cache : v_cache;
   }

@@ -12,7 +12,7 @@ namespace {
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-swiglu_kernel(const T* __restrict__ upgate, const PeerOut out, int64_t rows, int64_t width_vecs, int64_t in_ld) {
+swiglu_kernel(const T* upgate, const PeerOut out, int64_t rows, int64_t width_vecs, int64_t in_ld) {
   constexpr int E = Elem<T>::kPerVec;
   pdl_launch_dependents();
   pdl_wait();  // upgate is the preceding kernel's output
@@ -21,8 +21,8 @@ swiglu_kernel(const T* __restrict__ upgate, const PeerOut out, int64_t rows, int
     const int64_t r = i / width_vecs, v = i - r * width_vecs;
     const T* row = upgate + r * in_ld;
     float up[E], gate[E], res[E];
-    unpack16<T>(ld_stream16(row + v * E), up);
-    unpack16<T>(ld_stream16(row + (width_vecs + v) * E), gate);
+    unpack16<T>(ld_ordered_stream16(row + v * E), up);
+    unpack16<T>(ld_ordered_stream16(row + (width_vecs + v) * E), gate);
 #pragma unroll
     for (int e = 0; e < E; ++e) res[e] = __fmul_rn(__fdiv_rn(gate[e], __fadd_rn(1.0f, expf(-gate[e]))), up[e]);
     const U4 packed = pack16<T>(res);
@@ -34,7 +34,7 @@ swiglu_kernel(const T* __restrict__ upgate, const PeerOut out, int64_t rows, int
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-swiglu_scalar_kernel(const T* __restrict__ upgate, const PeerOut out, int64_t rows, int64_t width, int64_t in_ld) {
+swiglu_scalar_kernel(const T* upgate, const PeerOut out, int64_t rows, int64_t width, int64_t in_ld) {
   pdl_launch_dependents();
   pdl_wait();
   const int64_t total = rows * width;

@@ -1046,16 +1046,26 @@ w4a16_mma_kernel(W4Args a, int col_groups) {
   fetch(buf0, cta_col0, 0);  // the first batch's weights go out before x is staged
   pdl_wait();                // x may be the preceding kernel's output; the weights are not
 
-  const int units = a.k / 8;
-  for (int i = threadIdx.x; i < a.m * units; i += kThreads) {
-    const int r = i / units, u = i - r * units;
-    const U4 v = ld_cached16(a.x + static_cast<size_t>(r) * a.k + u * 8);
-    U4 o;  // k 0..7 -> 0,4,1,5,2,6,3,7: the pairs the unpack produces
-    o.x = __byte_perm(v.x, v.z, 0x5410);
-    o.y = __byte_perm(v.x, v.z, 0x7632);
-    o.z = __byte_perm(v.y, v.w, 0x5410);
-    o.w = __byte_perm(v.y, v.w, 0x7632);
-    *reinterpret_cast<U4*>(xs + static_cast<size_t>(r) * pitch + u * 16) = o;
+  const int units = a.k / 8, x_units = a.m * units;
+  constexpr int kXFlight = 8;  // ordered loads in flight per thread
+  const uint32_t per_unit = 0xffffffffu / units + 1;  // i / units = the high word of i * per_unit, for i * units below 2^32
+  for (int i0 = threadIdx.x; i0 < x_units; i0 += kXFlight * kThreads) {
+    U4 v[kXFlight];
+#pragma unroll
+    for (int j = 0; j < kXFlight; ++j)
+      v[j] = ld_ordered16_if(a.x + static_cast<size_t>(i0 + j * kThreads) * 8, i0 + j * kThreads < x_units);
+#pragma unroll
+    for (int j = 0; j < kXFlight; ++j) {
+      const int i = i0 + j * kThreads, r = static_cast<int>(__umulhi(i, per_unit));
+      if (i < x_units) {
+        U4 o;  // k 0..7 -> 0,4,1,5,2,6,3,7: the pairs the unpack produces
+        o.x = __byte_perm(v[j].x, v[j].z, 0x5410);
+        o.y = __byte_perm(v[j].x, v[j].z, 0x7632);
+        o.z = __byte_perm(v[j].y, v[j].w, 0x5410);
+        o.w = __byte_perm(v[j].y, v[j].w, 0x7632);
+        *reinterpret_cast<U4*>(xs + (i + r) * 16) = o;  // 16 bytes of pad behind every row
+      }
+    }
   }
   __syncthreads();
   // this lane's B fragments: row n of x; lanes past M read row 0 and feed output rows that are never stored
