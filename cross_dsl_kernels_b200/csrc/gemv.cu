@@ -704,9 +704,9 @@ extern "C" size_t xdk_gemv_scratch_bytes(int64_t m, int64_t k, int64_t n, int we
 
 extern "C" int xdk_gemv_f32(const float* x, const float* w, const float* bias, float* y, int64_t m, int64_t k,
                             int64_t n, int weight_is_nk, int split_k, void* scratch, size_t scratch_bytes, void* stream) {
-  // version 1 semantics: passing scratch asks for strict FP32 arithmetic
-  return xdk_gemv_f32_v2(x, w, bias, y, m, k, n, weight_is_nk, split_k, scratch, scratch_bytes, scratch ? XDK_STRICT_FP32 : 0u,
-                         stream);
+  // version 1 semantics: passing scratch asks for strict FP32 arithmetic, and more than 16 rows always had it
+  return xdk_gemv_f32_v2(x, w, bias, y, m, k, n, weight_is_nk, split_k, scratch, scratch_bytes,
+                         scratch || m > 16 ? XDK_STRICT_FP32 : 0u, stream);
 }
 
 extern "C" int xdk_gemv_f32_v2(const float* x, const float* w, const float* bias, float* y, int64_t m, int64_t k,
@@ -733,8 +733,8 @@ extern "C" int xdk_gemv_f32_peer(const float* x, const float* w, const float* bi
   if (int st = require_sm100()) return st;
   const bool nk = weight_is_nk != 0;
 
-  // More than 16 rows unless strict FP32 was asked for: the mma.sync split-TF32 kernel (gemv_mma.cu, with both sides' times
-  // and errors).  It would also be faster than the tcgen05 kernel for 5 .. 8 rows of a wide [K, N] matrix (N = 11012 41 us
+  // More than 16 rows of a long K unless strict FP32 was asked for: the mma.sync split-TF32 kernel (gemv_mma.cu, with both
+  // sides' times and errors).  It would also be faster than the tcgen05 kernel for 5 .. 8 rows of a wide [K, N] matrix (N = 11012 41 us
   // against 50), but not for 16 (N = 14336 60 / 50), and a row keeps its bits whatever the batch of up to 16 it is in.
   if (split_k == 0 && !strict && m > 16 && gemv_mma_eligible(x, w, m, k, n, nk))
     return launch_gemv_mma(x, w, bias, y, static_cast<int>(m), static_cast<int>(k), static_cast<int>(n), nk, static_cast<cudaStream_t>(stream));

@@ -1,15 +1,21 @@
-// FP32 projection of more than 16 rows on mma.sync (tf32), with the accuracy of FP32 FMAs.
+// FP32 projection of more than 16 rows and a long K on mma.sync (tf32), with the accuracy of FP32 FMAs.
 //
 // y[M, N] = x[M, K] . W + bias.  Both operands are split into two TF32 numbers, v = hi + lo (hi = v rounded to
 // TF32's 11 significant bits, lo = v - hi, exact and of either sign), and the product is hi.hi + hi.lo + lo.hi.  The tensor
 // core truncates as it accumulates, so an accumulator only takes the six MMAs of 16 k, the small products first, before it
-// is added to an FP32 sum with rounding.  Relative L2 error against 64 bits at K = 4096 / 14336: 1.6e-7 / 2.3e-7, the
-// FP32-FMA kernels' 1.6e-7 .. 2.9e-7 (with hi cut off instead of rounded 5.7e-7, in another order of the products 1.9e-7).
+// is added to an FP32 sum with rounding.  What the products lose (the last bit of an operand, lo.lo, the truncation) is about
+// 1e-7 at any K, the sum's own error grows with K as that of FMAs does: so the kernel only takes shapes where it is no less
+// accurate than the FP32-FMA kernels that had them.  Relative L2 error against 64 bits, e-7, here / FMAs, normal operands:
+//   [K, N]  K = 128 1.17 / 0.93, 1024 1.29 / 1.25, 2048 1.40 / 1.31, 4096 1.57 / 1.65, 8192 1.87 / 2.18, 14336 2.25 / 2.80
+//   [N, K]  N <= 2368, where FMAs split K four ways or eight: 4096 1.58 / 1.27, 14336 2.26 / 2.04
+//           wider, two ways: 1024 1.29 / 1.00, 2048 1.39 / 1.22, 4096 1.57 / 1.59, 8192 1.87 / 2.14, 14336 2.25 / 2.77
+// (With hi cut off instead of rounded 5.7 at K = 4096, in another order of the products 1.9.)  Operands of one sign: 0.87 at
+// K = 4096, 1.01 at 14336; FMAs 0.45 .. 0.6.
 // An infinity does not split (lo = inf - inf): an output that is not finite is computed again with FMAs.
 //
 // Times, us, against the kernels that had the shapes before (K = 4096 unless said): M = 64, N = 4096 61 against 89 .. 94
 // (FP32 FMAs of a 16 x 4 register tile, W walked once per 16 rows), M = 64, N = 14336 203 / 266 .. 281, M = 64, K = 14336,
-// N = 4096 190 / 267 .. 290, M = 24, K = 1024, N = 2048 10 / 15 .. 22.  What bounds it: with one CTA of eight warps an SM,
+// N = 4096 190 / 267 .. 290.  What bounds it: with one CTA of eight warps an SM,
 // latency -- the tensor pipe would need 22 us for M = 64, N = 4096.
 //
 // The loop is built round the stream of W.  A CTA (one per SM) owns up to 16 rows and 16 G columns over all of its K; its
@@ -304,6 +310,8 @@ int launch_mma(const MmaArgs& a, int ctas, int ranks, cudaStream_t stream) {
 }  // namespace
 
 bool gemv_mma_eligible(const float* x, const float* w, int64_t m, int64_t k, int64_t n, bool nk) {
+  // the least K, and for [N, K] the least N, at which the error is no larger than that of FMAs (figures above)
+  if (k < 4096 || (nk && n <= 2368)) return false;
   return m >= 1 && m <= 16 * 65535LL && k % 4 == 0 && (nk || n % 4 == 0) && aligned16(x) && aligned16(w) && k < (1 << 30) && n < (1 << 30);
 }
 

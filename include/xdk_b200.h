@@ -51,8 +51,9 @@ typedef enum xdk_dtype {
  * version-1 namesake plus `unsigned flags` before the stream; the version-1 functions stay and behave
  * as before.
  *   XDK_STRICT_FP32       (xdk_gemv_f32_v2 only) every product and sum is an FP32 FMA on the CUDA cores;
- *                         without it a large 4 < M <= 16 projection may run on the tensor cores as
- *                         split-TF32 products (inside the projection's 1e-5 gate, not bit-identical).
+ *                         without it a large 4 < M <= 16 projection, and one of M > 16 rows with
+ *                         K >= 4096, may run on the tensor cores as split-TF32 products (inside the
+ *                         projection's 1e-5 gate, not bit-identical).
  *                         The choice of arithmetic never depends on whether scratch was passed.
  *   XDK_DEPENDENT_LAUNCH  the kernel is launched as a programmatic dependent of the preceding kernel
  *                         of the stream: it is scheduled while that kernel drains, and waits for that
@@ -136,7 +137,7 @@ XDK_API int xdk_rmsnorm_v2(const void* x, const void* residual, const void* weig
  *     K*N >= 4M) runs on the tensor cores: every operand is split into two TF32 numbers and
  *     the product formed as hi*hi + hi*lo + lo*hi with FP32 accumulation.  Against an FP64 product
  *     the relative L2 error is ~3e-6 (8e-6 on all-positive operands), below the projection's gate (1e-5), for
- *     every K the path takes (other rows stay on FP32 FMAs), but it is not the FP32-FMA result bit for bit, and
+ *     every K the path takes, but it is not the FP32-FMA result bit for bit, and
  *     an infinity in x or W yields NaN where FP32 FMAs yield an infinity (lo = v - hi is NaN for v = inf).
  *     Other shapes use the cluster kernels.
  *   scratch != NULL (device memory, >= xdk_gemv_scratch_bytes(...), 16-byte aligned, written and
@@ -144,7 +145,7 @@ XDK_API int xdk_rmsnorm_v2(const void* x, const void* residual, const void* weig
  *     persistent tile-stream kernel that deals the weight tiles evenly to all SMs.  Calls that
  *     share one scratch buffer must not overlap on the GPU.
  * Results are deterministic for a given (shape, split_k, scratch or not).  bias may be NULL.
- * M, K, N >= 1; M > 16 is processed in row tiles of 16 (the weight stream repeats per tile).
+ * M, K, N >= 1; M > 16 is processed in row tiles of 16 (the weight stream repeats per tile) by FP32 FMAs.
  * Replaces decode_gemv / decode_gemv_warp / decode_gemv_rows
  * (csrc/gemv/gemv_ext.cpp:57-85), decode_gemv_simt_{warp,rows} and
  * decode_gemm_tiled (csrc/gemv/gemv_simt_ext.cpp:49-83); split-K semantics as
@@ -157,7 +158,12 @@ XDK_API int xdk_gemv_f32(const float* x, const float* w, const float* bias, floa
  * Version 2: the arithmetic is chosen by `flags`, not by the scratch pointer.  With XDK_STRICT_FP32 the
  * call never leaves FP32 FMA arithmetic; scratch (optional, same rules as above) then only lets a large
  * 4 < M <= 16 projection (K*N >= 48M) use the balanced tile-stream kernel instead of the cluster
- * kernels.  Without the flag, scratch is ignored whenever the tensor-core kernel takes the shape.
+ * kernels.  Without the flag, scratch is ignored whenever a tensor-core kernel takes the shape.
+ * Without the flag and with split_k = 0, M > 16 rows with K >= 4096, K % 4 == 0, 16-byte aligned x and w, and N % 4 == 0
+ * (KN weights) or N > 2368 (NK weights) also run on the tensor cores: split-TF32 products whose relative L2 error against an
+ * FP64 product is no larger than that of the FP32 FMAs they replace (1.6e-7 at K = 4096, 2.3e-7 at 14336; about 1e-7, twice
+ * the FMAs', on operands of one sign).  An output that comes out not finite is computed again with FP32 FMAs, so infinities and NaNs
+ * are those of the plain products.  XDK_STRICT_FP32, or version 1, keeps FP32 FMAs.
  */
 XDK_API int xdk_gemv_f32_v2(const float* x, const float* w, const float* bias, float* y,
                     int64_t m, int64_t k, int64_t n, int weight_is_nk, int split_k,
