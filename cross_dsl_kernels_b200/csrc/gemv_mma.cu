@@ -15,7 +15,9 @@
 //
 // Times, us, against the kernels that had the shapes before (K = 4096 unless said): M = 64, N = 4096 61 against 89 .. 94
 // (FP32 FMAs of a 16 x 4 register tile, W walked once per 16 rows), M = 64, N = 14336 203 / 266 .. 281, M = 64, K = 14336,
-// N = 4096 190 / 267 .. 290.  What bounds it: with one CTA of eight warps an SM,
+// N = 4096 190 / 267 .. 290; M = 592 434 / 765, M = 1200 1137 / 1541, M = 5000 3903 / 6396 (N = 4096, [K, N]; [N, K] alike).  Narrow [K, N]:
+// N = 768, M = 17 16 / 17, M = 64 21 / 31, M = 1200 283 / 524, but N = 512, M = 17 .. 48 17 .. 22 / 14 .. 17, N = 256, M = 64 18 / 12: a
+// block of rows has too few column groups there.  What bounds it: with one CTA of eight warps an SM,
 // latency -- the tensor pipe would need 22 us for M = 64, N = 4096.
 //
 // The loop is built round the stream of W.  A CTA (one per SM) owns up to 16 rows and 16 G columns over all of its K; its
@@ -48,6 +50,7 @@ struct MmaArgs {
   int m, k, n;
   int groups;  // of 16 columns
   int k_rank;  // k per CTA of a cluster (a multiple of kStepK)
+  int block0;  // first block of 16 rows of this launch
 };
 
 __device__ __forceinline__ void cp_async16_or_zero(void* dst, const void* src, bool live) {
@@ -101,7 +104,7 @@ gemv_mma_kernel(MmaArgs a) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i = lane >> 2, q = lane & 3;
   const int ranks = gridDim.y, rank = blockIdx.y;
-  const int row0 = blockIdx.z * 16, rows = min(16, a.m - row0);  // more than 16 rows: blocks of them, W comes from L2
+  const int row0 = (a.block0 + blockIdx.z) * 16, rows = min(16, a.m - row0);  // blocks of rows: W comes from L2 for all but one
   const int k_begin = rank * a.k_rank, k_end = min(a.k, k_begin + a.k_rank);
   const int all_steps = k_begin < k_end ? (k_end - k_begin + kStepK - 1) / kStepK : 0;
   const int steps = all_steps > warp ? (all_steps - warp + kWarps - 1) / kWarps : 0;  // of this warp: warp, warp + 8, ...
@@ -290,28 +293,29 @@ gemv_mma_kernel(MmaArgs a) {
 }
 
 template <bool NK, int MR, int G>
-int launch_mma(const MmaArgs& a, int ctas, int ranks, cudaStream_t stream) {
+int launch_mma(const MmaArgs& a, int ctas, int ranks, int blocks, cudaStream_t stream) {
   constexpr size_t smem = Ring<NK, G>::bytes(MR);
   static_assert(smem <= 227 * 1024, "one CTA per SM");
   auto kernel = gemv_mma_kernel<NK, MR, G>;
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (err != cudaSuccess) return note_launch(err);
-  return launch_opts(kernel, dim3(ctas, ranks, (a.m + 15) / 16), dim3(kThreads), smem, stream, static_cast<unsigned>(ranks),
+  return launch_opts(kernel, dim3(ctas, ranks, blocks), dim3(kThreads), smem, stream, static_cast<unsigned>(ranks),
                      (call_flags() & XDK_DEPENDENT_LAUNCH) != 0, a);
 }
 template <bool NK, int MR>
-int launch_mma(const MmaArgs& a, int ctas, int ranks, cudaStream_t stream) {
+int launch_mma(const MmaArgs& a, int ctas, int ranks, int blocks, cudaStream_t stream) {
   const int per = (a.groups + ctas - 1) / ctas;  // column groups of the busiest CTA
-  if (per <= 2) return launch_mma<NK, MR, 2>(a, ctas, ranks, stream);
-  if (per <= 4) return launch_mma<NK, MR, 4>(a, ctas, ranks, stream);
-  return launch_mma<NK, MR, 8>(a, ctas, ranks, stream);
+  if (per <= 2) return launch_mma<NK, MR, 2>(a, ctas, ranks, blocks, stream);
+  if (per <= 4) return launch_mma<NK, MR, 4>(a, ctas, ranks, blocks, stream);
+  return launch_mma<NK, MR, 8>(a, ctas, ranks, blocks, stream);
 }
 
 }  // namespace
 
 bool gemv_mma_eligible(const float* x, const float* w, int64_t m, int64_t k, int64_t n, bool nk) {
-  // the least K, and for [N, K] the least N, at which the error is no larger than that of FMAs (figures above)
-  if (k < 4096 || (nk && n <= 2368)) return false;
+  // the least K, and for [N, K] the least N, at which the error is no larger than that of FMAs, and for [K, N] the least N at
+  // which it is no slower at any M (figures above)
+  if (k < 4096 || n <= (nk ? 2368 : 764)) return false;
   return m >= 1 && m <= 16 * 65535LL && k % 4 == 0 && (nk || n % 4 == 0) && aligned16(x) && aligned16(w) && k < (1 << 30) && n < (1 << 30);
 }
 
@@ -320,13 +324,23 @@ int launch_gemv_mma(const float* x, const float* w, const float* bias, const Pee
   MmaArgs a;
   a.x = x, a.w = w, a.bias = bias, a.out = y, a.m = m, a.k = k, a.n = n;
   a.groups = (n + 15) / 16;
-  const int slabs = (m + 15) / 16, sms = max(1, sm_count() / slabs);  // SMs a block of 16 rows can have
-  // fewer column groups than SMs: share K between the CTAs of a cluster, as long as each keeps a few steps per warp
-  int ranks = 1;
-  while (ranks < 8 && a.groups * ranks * 2 <= sms && k / (ranks * 2) >= 4 * kStepK * kWarps) ranks *= 2;
+  const int sms = sm_count();
+  // Few column groups: two CTAs of a cluster share K.  By N alone: the order of the sums, and with it the bits of a row, do not
+  // depend on how many rows there are.
+  const int ranks = a.groups * 2 <= sms ? 2 : 1;
   a.k_rank = ((k + ranks - 1) / ranks + kStepK - 1) / kStepK * kStepK;
-  const int ctas = a.groups < sms / ranks ? a.groups : sms / ranks;
-  return nk ? launch_mma<true, 2>(a, ctas, ranks, stream) : launch_mma<false, 2>(a, ctas, ranks, stream);
+  // A block of 16 rows gets an equal share of the SMs, in whole CTAs.  Many rows go in several launches of blocks that have at
+  // least four CTAs each: the fewer there are, the more SMs the rounding leaves idle (1200 rows in one launch had 75 CTAs).
+  const int blocks = (m + 15) / 16, most = sms > 4 ? sms / 4 : 1;
+  const int launches = (blocks + most - 1) / most;
+  for (int i = 0; i < launches; ++i) {
+    a.block0 = static_cast<int>(static_cast<int64_t>(i) * blocks / launches);
+    const int count = static_cast<int>(static_cast<int64_t>(i + 1) * blocks / launches) - a.block0;
+    const int share = sms / (count * ranks), ctas = a.groups < share ? a.groups : (share > 1 ? share : 1);
+    const int st = nk ? launch_mma<true, 2>(a, ctas, ranks, count, stream) : launch_mma<false, 2>(a, ctas, ranks, count, stream);
+    if (st != XDK_OK) return st;
+  }
+  return XDK_OK;
 }
 
 }  // namespace xdk

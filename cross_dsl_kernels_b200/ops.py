@@ -87,7 +87,7 @@ def decode_linear(x, weight, bias=None, *, out_dtype=None, weight_layout: str = 
 
     With ``split_k=0`` and 4 < M <= 16 a large projection runs on the tensor cores as split-TF32
     products with FP32 accumulation (relative L2 error ~1e-6 against an FP64 product, inside the
-    projection's 1e-5 gate), and so does M > 16 with K >= 4096 (N > 2368 for "NK" weights), where the
+    projection's 1e-5 gate), and so does M > 16 with K >= 4096 (N >= 768 for "KN", > 2368 for "NK" weights), where the
     error is no larger than that of FP32 FMAs (1.6e-7 at K = 4096).  ``strict_fp32=True`` keeps such
     shapes on the CUDA cores, where every product and sum is an FP32 FMA; 4 < M <= 16 then needs a
     scratch block per call.

@@ -45,7 +45,7 @@ def test_operands_that_do_not_split(layout):
 
 
 @pytest.mark.parametrize("layout,k,n,split", [("KN", 4096, 1024, True), ("KN", 14336, 4100, True), ("NK", 4096, 2372, True),
-                                              ("NK", 8192, 4096, True), ("KN", 4092, 1024, False), ("KN", 64, 512, False),
+                                              ("NK", 8192, 4096, True), ("KN", 4096, 768, True), ("KN", 4096, 764, False), ("KN", 4092, 1024, False), ("KN", 64, 512, False),
                                               ("NK", 4096, 2368, False), ("NK", 2048, 4096, False), ("NK", 4, 8, False)])
 def test_the_split_is_no_less_accurate_than_fp32_fmas(layout, k, n, split):
     """More than 16 rows: split-TF32 products where their error against 64 bits is no larger than that of the FP32 FMAs, the bits of
@@ -65,3 +65,17 @@ def test_the_split_is_no_less_accurate_than_fp32_fmas(layout, k, n, split):
                                                  None, 0, _native.stream_ptr(x.device)), "version 1")
         assert torch.equal(first, strict)
     assert ours <= fmas * 1.01  # means of four draws of 24 N outputs: they scatter by less than 1 %
+
+
+@pytest.mark.parametrize("layout,k,n", [("KN", 4096, 768), ("KN", 4100, 1028), ("KN", 8192, 1200), ("KN", 4096, 512), ("NK", 4096, 2400)])
+def test_the_bits_of_a_row_do_not_depend_on_the_rows_beside_it(layout, k, n):
+    """More than 16 rows, up to several launches of them: the same bits for a row in every batch, and the right ones."""
+    from cross_dsl_kernels_b200.ops import decode_linear
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x, w = torch.randn(1300, k, generator=g, device="cuda"), torch.randn(k, n, generator=g, device="cuda") / k ** 0.5
+    weight, bias = w if layout == "KN" else w.t().contiguous(), torch.randn(n, generator=g, device="cuda")
+    whole = decode_linear(x, weight, bias, weight_layout=layout)
+    assert rel_l2(whole, x.double() @ w.double() + bias.double()) <= 2e-7 * (k / 4096) ** 0.5  # 1.6e-7 of the product, and the bias's sum
+    for m in (17, 32, 33, 64, 100, 288, 289, 592, 593, 1185):
+        assert torch.equal(decode_linear(x[:m], weight, bias, weight_layout=layout), whole[:m])
+        assert torch.equal(decode_linear(x[1300 - m:], weight, bias, weight_layout=layout), whole[1300 - m:])
