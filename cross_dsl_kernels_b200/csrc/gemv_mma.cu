@@ -11,11 +11,13 @@
 //           wider, two ways: 1024 1.29 / 1.00, 2048 1.39 / 1.22, 4096 1.57 / 1.59, 8192 1.87 / 2.14, 14336 2.25 / 2.77
 // (With hi cut off instead of rounded 5.7 at K = 4096, in another order of the products 1.9.)  Operands of one sign: 0.87 at
 // K = 4096, 1.01 at 14336; FMAs 0.45 .. 0.6.
-// An infinity does not split (lo = inf - inf): an output that is not finite is computed again with FMAs.
+// An infinity does not split (lo = inf - inf): a pass with a sum that is not finite is done once more, with a split that carries
+// infinities and NaNs in its leading product alone (us for M = 64, K = N = 4096 and a NaN in every row of x, [K, N] / [N, K]: 224 / 221;
+// with a thread that went through K for each such output 1669 / 4004).
 //
-// Times, us, against the kernels that had the shapes before (K = 4096 unless said): M = 64, N = 4096 61 against 89 .. 94
-// (FP32 FMAs of a 16 x 4 register tile, W walked once per 16 rows), M = 64, N = 14336 203 / 266 .. 281, M = 64, K = 14336,
-// N = 4096 190 / 267 .. 290; M = 592 434 / 765, M = 1200 1137 / 1541, M = 5000 3903 / 6396 (N = 4096, [K, N]; [N, K] alike).  Narrow [K, N]:
+// Times, us, against the kernels that had the shapes before (K = 4096 unless said): M = 64, N = 4096 57 .. 60 against 89 .. 94
+// (FP32 FMAs of a 16 x 4 register tile, W walked once per 16 rows), M = 64, N = 14336 200 / 266 .. 281, M = 64, K = 14336,
+// N = 4096 174 .. 187 / 267 .. 290; M = 592 426 / 765, M = 1200 1137 / 1541, M = 5000 3903 / 6396 (N = 4096, [K, N]; [N, K] alike).  Narrow [K, N]:
 // N = 768, M = 17 16 / 17, M = 64 21 / 31, M = 1200 283 / 524, but N = 512, M = 17 .. 48 17 .. 22 / 14 .. 17, N = 256, M = 64 18 / 12: a
 // block of rows has too few column groups there.  What bounds it: with one CTA of eight warps an SM,
 // latency -- the tensor pipe would need 22 us for M = 64, N = 4096.
@@ -31,6 +33,8 @@
 // The warps' sums meet in shared memory in warp order.  A narrow matrix splits K over the CTAs of a cluster, whose sums
 // are added in rank order through distributed shared memory.  Deterministic.
 #include <cooperative_groups.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -61,25 +65,30 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 struct Split {
-  uint32_t hi, lo;
+  uint32_t hi, lo, lead;  // lead: the factor of the leading product, hi but for what does not split
 };
 __device__ __forceinline__ Split split_tf32(float v) {
   const uint32_t hi = (__float_as_uint(v) + 0x1000u) & 0xffffe000u;
-  return Split{hi, __float_as_uint(__fsub_rn(v, __uint_as_float(hi)))};
+  return Split{hi, __float_as_uint(__fsub_rn(v, __uint_as_float(hi))), hi};
+}
+// The same parts of what splits.  An infinity or a NaN is in the leading product only, whose outcome is then that of the plain
+// product; a value that would round up to infinity is cut off instead, and one that would round to zero is kept apart from it.
+__device__ __forceinline__ Split split_any(float v) {
+  const uint32_t bits = __float_as_uint(v), size = bits & 0x7fffffffu;
+  if (size >= 0x7f800000u) return Split{0u, 0u, size > 0x7f800000u ? 0x7fffffffu : bits};
+  uint32_t hi = (bits + 0x1000u) & 0xffffe000u;
+  if ((hi & 0x7fffffffu) == 0x7f800000u) hi = bits & 0xffffe000u;
+  if ((hi & 0x7fffffffu) == 0u && size != 0u) hi |= 0x2000u;
+  return Split{hi, __float_as_uint(__fsub_rn(v, __uint_as_float(hi))), hi};
+}
+template <bool ANY>
+__device__ __forceinline__ Split split(float v) {
+  return ANY ? split_any(v) : split_tf32(v);
 }
 __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// One output with FP32 FMAs, for the operands the split cannot carry (infinity: lo = inf - inf).
-template <bool NK>
-__device__ __noinline__ float plain_dot(const MmaArgs& a, int row, int col) {
-  float v = 0.0f;
-  for (int k = 0; k < a.k; ++k)
-    v = fmaf(a.x[static_cast<size_t>(row) * a.k + k], NK ? a.w[static_cast<size_t>(col) * a.k + k] : a.w[static_cast<size_t>(k) * a.n + col], v);
-  return v;
 }
 
 template <bool NK, int G>
@@ -169,121 +178,130 @@ gemv_mma_kernel(MmaArgs a) {
     };
 
     float sum[G][MR][4];
+    auto multiply = [&](auto any) {  // any: operands that do not split
+      constexpr bool ANY = decltype(any)::value;
 #pragma unroll
-    for (int g = 0; g < G; ++g)
+      for (int g = 0; g < G; ++g)
 #pragma unroll
-      for (int r = 0; r < MR; ++r)
+        for (int r = 0; r < MR; ++r)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) sum[g][r][e] = 0.0f;
-    float xn[MR][4];
-    for (int s = 0; s < D - 1; ++s) fetch(s);
-    fetch_x(0, xn);
-    for (int s = 0; s < steps; ++s) {
-      Split xs[MR][4];
+          for (int e = 0; e < 4; ++e) sum[g][r][e] = 0.0f;
+      float xn[MR][4];
+      for (int s = 0; s < D - 1; ++s) fetch(s);
+      fetch_x(0, xn);
+      for (int s = 0; s < steps; ++s) {
+        Split xs[MR][4];
 #pragma unroll
-      for (int r = 0; r < MR; ++r)
+        for (int r = 0; r < MR; ++r)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) xs[r][e] = split_tf32(xn[r][e]);
-      cp_async_wait<D - 2>();
-      __syncwarp();  // the step has landed for every lane, and every lane has read the slot that is refilled now
-      fetch(s + D - 1);
-      fetch_x(s + 1, xn);
-      const float* tile = ring + (s % D) * R::kStage;
+          for (int e = 0; e < 4; ++e) xs[r][e] = split<ANY>(xn[r][e]);
+        cp_async_wait<D - 2>();
+        __syncwarp();  // the step has landed for every lane, and every lane has read the slot that is refilled now
+        fetch(s + D - 1);
+        fetch_x(s + 1, xn);
+        const float* tile = ring + (s % D) * R::kStage;
 #pragma unroll
-      for (int g = 0; g < G; g += 2) {  // two groups at a time: twice the independent MMA chains
-        if (g >= ng) break;             // (an odd last group is paired with columns whose sums are not stored)
-        float w[2][2][4];               // [group][column i, column i + 8 of the MMA][slot]
+        for (int g = 0; g < G; g += 2) {  // two groups at a time: twice the independent MMA chains
+          if (g >= ng) break;             // (an odd last group is paired with columns whose sums are not stored)
+          float w[2][2][4];               // [group][column i, column i + 8 of the MMA][slot]
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (NK) {
-            const float4 t0 = *reinterpret_cast<const float4*>(tile + ((g + h) * 16 + i) * R::kPitch + q * 4);
-            const float4 t1 = *reinterpret_cast<const float4*>(tile + ((g + h) * 16 + i + 8) * R::kPitch + q * 4);
-            w[h][0][0] = t0.x, w[h][0][1] = t0.y, w[h][0][2] = t0.z, w[h][0][3] = t0.w;
-            w[h][1][0] = t1.x, w[h][1][1] = t1.y, w[h][1][2] = t1.z, w[h][1][3] = t1.w;
-          } else {
+          for (int h = 0; h < 2; ++h) {
+            if (NK) {
+              const float4 t0 = *reinterpret_cast<const float4*>(tile + ((g + h) * 16 + i) * R::kPitch + q * 4);
+              const float4 t1 = *reinterpret_cast<const float4*>(tile + ((g + h) * 16 + i + 8) * R::kPitch + q * 4);
+              w[h][0][0] = t0.x, w[h][0][1] = t0.y, w[h][0][2] = t0.z, w[h][0][3] = t0.w;
+              w[h][1][0] = t1.x, w[h][1][1] = t1.y, w[h][1][2] = t1.z, w[h][1][3] = t1.w;
+            } else {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float2 t = *reinterpret_cast<const float2*>(tile + (q + e * 4) * R::kPitch + (g + h) * 16 + i * 2);
-              w[h][0][e] = t.x, w[h][1][e] = t.y;
+              for (int e = 0; e < 4; ++e) {
+                const float2 t = *reinterpret_cast<const float2*>(tile + (q + e * 4) * R::kPitch + (g + h) * 16 + i * 2);
+                w[h][0][e] = t.x, w[h][1][e] = t.y;
+              }
             }
           }
-        }
-        float acc[2][MR][4];
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int r = 0; r < MR; ++r)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[h][r][e] = 0.0f;
-        uint32_t hi[2][2][4], lo[2][2][4];  // [MMA j: slots 2 j and 2 j + 1][group][fragment register]
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
+          float acc[2][MR][4];
 #pragma unroll
           for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const Split v = split_tf32(w[h][e & 1][2 * j + (e >> 1)]);
-              hi[j][h][e] = v.hi, lo[j][h][e] = v.lo;
-            }
-        // the small products first: what the tensor core truncates off an accumulator then only counts for the last two
+            for (int r = 0; r < MR; ++r)
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+              for (int e = 0; e < 4; ++e) acc[h][r][e] = 0.0f;
+          uint32_t hi[2][2][4], lo[2][2][4], lead[2][2][4];  // [MMA j: slots 2 j and 2 j + 1][group][fragment register]
 #pragma unroll
-          for (int r = 0; r < MR; ++r)
+          for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int h = 0; h < 2; ++h) mma_tf32(acc[h][r], lo[j][h], xs[r][2 * j].hi, xs[r][2 * j + 1].hi);
+            for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+              for (int e = 0; e < 4; ++e) {
+                const Split v = split<ANY>(w[h][e & 1][2 * j + (e >> 1)]);
+                hi[j][h][e] = v.hi, lo[j][h][e] = v.lo, lead[j][h][e] = v.lead;
+              }
+          // the small products first: what the tensor core truncates off an accumulator then only counts for the last two
 #pragma unroll
-          for (int r = 0; r < MR; ++r)
+          for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int h = 0; h < 2; ++h) mma_tf32(acc[h][r], hi[j][h], xs[r][2 * j].lo, xs[r][2 * j + 1].lo);
+            for (int r = 0; r < MR; ++r)
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+              for (int h = 0; h < 2; ++h) mma_tf32(acc[h][r], lo[j][h], xs[r][2 * j].hi, xs[r][2 * j + 1].hi);
 #pragma unroll
-          for (int r = 0; r < MR; ++r)
+          for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int h = 0; h < 2; ++h) mma_tf32(acc[h][r], hi[j][h], xs[r][2 * j].hi, xs[r][2 * j + 1].hi);
+            for (int r = 0; r < MR; ++r)
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+              for (int h = 0; h < 2; ++h) mma_tf32(acc[h][r], hi[j][h], xs[r][2 * j].lo, xs[r][2 * j + 1].lo);
 #pragma unroll
-          for (int r = 0; r < MR; ++r)
+          for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) sum[g + h][r][e] = __fadd_rn(sum[g + h][r][e], acc[h][r][e]);
-      }
-    }
-    cp_async_wait<0>();
-    __syncthreads();  // the rings are done with: their memory takes the sums, [warp][row][column of the pass]
+            for (int r = 0; r < MR; ++r)
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      if (g >= ng) break;
+              for (int h = 0; h < 2; ++h) mma_tf32(acc[h][r], lead[j][h], xs[r][2 * j].lead, xs[r][2 * j + 1].lead);
 #pragma unroll
-      for (int r = 0; r < MR; ++r)
+          for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {  // rows 2 q + (e & 1) of x, column i (e < 2) or i + 8 of the MMA
-          const int row = r * 8 + q * 2 + (e & 1);
-          const int col = g * 16 + (NK ? i + (e >> 1) * 8 : i * 2 + (e >> 1));
-          smem[(warp * 8 * MR + row) * R::kSumPitch + col] = sum[g][r][e];
+            for (int r = 0; r < MR; ++r)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) sum[g + h][r][e] = __fadd_rn(sum[g + h][r][e], acc[h][r][e]);
         }
-    }
-    __syncthreads();
+      }
+    };
     const int cols = ng * 16, outs = rows * cols;
-    for (int o = threadIdx.x; o < outs; o += kThreads) {
-      const int row = o / cols, at = row * R::kSumPitch + (o - row * cols);
-      float v = smem[at];
+    for (bool again = false;;) {  // once more if a sum is not finite
+      if (again) multiply(std::true_type{});
+      else multiply(std::false_type{});
+      cp_async_wait<0>();
+      __syncthreads();  // the rings are done with: their memory takes the sums, [warp][row][column of the pass]
 #pragma unroll
-      for (int w = 1; w < kWarps; ++w) v = __fadd_rn(v, smem[w * 8 * MR * R::kSumPitch + at]);
-      smem[at] = v;
+      for (int g = 0; g < G; ++g) {
+        if (g >= ng) break;
+#pragma unroll
+        for (int r = 0; r < MR; ++r)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {  // rows 2 q + (e & 1) of x, column i (e < 2) or i + 8 of the MMA
+            const int row = r * 8 + q * 2 + (e & 1);
+            const int col = g * 16 + (NK ? i + (e >> 1) * 8 : i * 2 + (e >> 1));
+            smem[(warp * 8 * MR + row) * R::kSumPitch + col] = sum[g][r][e];
+          }
+      }
+      __syncthreads();
+      bool bad = false;
+      for (int o = threadIdx.x; o < outs; o += kThreads) {
+        const int row = o / cols, at = row * R::kSumPitch + (o - row * cols);
+        float v = smem[at];
+#pragma unroll
+        for (int w = 1; w < kWarps; ++w) v = __fadd_rn(v, smem[w * 8 * MR * R::kSumPitch + at]);
+        smem[at] = v;
+        bad |= !isfinite(v);
+      }
+      if (!__syncthreads_or(bad) || again) break;
+      again = true;
     }
     if (ranks > 1) cg::this_cluster().sync();  // every rank's sums stand in its shared memory
-    else __syncthreads();
     for (int o = threadIdx.x + rank * kThreads; o < outs; o += kThreads * ranks) {
       const int row = o / cols, c = o - row * cols;
       if (col0 + c >= a.n) continue;
       float* at = smem + row * R::kSumPitch + c;
       float v = ranks > 1 ? *cg::this_cluster().map_shared_rank(at, 0) : *at;
       for (int p = 1; p < ranks; ++p) v = __fadd_rn(v, *cg::this_cluster().map_shared_rank(at, p));  // rank order
-      if (!isfinite(v)) v = plain_dot<NK>(a, row0 + row, col0 + c);  // an operand that does not split, or a true overflow
       if (a.bias) v = __fadd_rn(v, a.bias[col0 + c]);
       peer_store(a.out, row0 + row, col0 + c, v);
     }

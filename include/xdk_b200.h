@@ -162,8 +162,8 @@ XDK_API int xdk_gemv_f32(const float* x, const float* w, const float* bias, floa
  * Without the flag and with split_k = 0, M > 16 rows with K >= 4096, K % 4 == 0, 16-byte aligned x and w, and N % 4 == 0,
  * N >= 768 (KN weights) or N > 2368 (NK weights) also run on the tensor cores: split-TF32 products whose relative L2 error against an
  * FP64 product is no larger than that of the FP32 FMAs they replace (1.6e-7 at K = 4096, 2.3e-7 at 14336; about 1e-7, twice
- * the FMAs', on operands of one sign).  An output that comes out not finite is computed again with FP32 FMAs, so infinities and NaNs
- * are those of the plain products.  Above 16 rows the bits of a row do not depend on how many there are.  XDK_STRICT_FP32, or version 1, keeps FP32 FMAs.
+ * the FMAs', on operands of one sign).  Where a sum comes out not finite it is taken again with a split that keeps infinities and
+ * NaNs whole, so they are those of the plain products.  Above 16 rows the bits of a row do not depend on how many there are.  XDK_STRICT_FP32, or version 1, keeps FP32 FMAs.
  */
 XDK_API int xdk_gemv_f32_v2(const float* x, const float* w, const float* bias, float* y,
                     int64_t m, int64_t k, int64_t n, int weight_is_nk, int split_k,

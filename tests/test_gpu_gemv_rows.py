@@ -79,3 +79,46 @@ def test_the_bits_of_a_row_do_not_depend_on_the_rows_beside_it(layout, k, n):
     for m in (17, 32, 33, 64, 100, 288, 289, 592, 593, 1185):
         assert torch.equal(decode_linear(x[:m], weight, bias, weight_layout=layout), whole[:m])
         assert torch.equal(decode_linear(x[1300 - m:], weight, bias, weight_layout=layout), whole[1300 - m:])
+
+
+@pytest.mark.parametrize("layout,n", [("KN", 772), ("KN", 1000), ("KN", 4100), ("KN", 20000), ("NK", 2380), ("NK", 20000)])
+def test_outputs_that_are_not_finite_at_full_size(layout, n):
+    """Rows of x and columns of W with infinities and NaNs, at every width of a pass: those outputs as FP32 FMAs give them, and for
+    the price of a second pass (they used to take one thread each, up to fifty times as long)."""
+    from cross_dsl_kernels_b200.ops import decode_linear
+    m, k = 70, 4096
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x, w = torch.randn(m, k, generator=g, device="cuda"), torch.randn(k, n, generator=g, device="cuda") / k ** 0.5
+    bias = torch.randn(n, generator=g, device="cuda")
+    clean = decode_linear(x, w if layout == "KN" else w.t().contiguous(), bias, weight_layout=layout)
+    x[3, 5], x[17, k - 1], x[m - 1, 0] = float("inf"), float("nan"), float("-inf")
+    x[20] *= 1e30  # times a column of 1e30: a true overflow
+    w[7, 2], w[9, n - 1] = float("nan"), float("inf")
+    w[:, 11] = 1e30
+    weight = w if layout == "KN" else w.t().contiguous()
+
+    def times(a, b):
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        decode_linear(a, b, bias, weight_layout=layout)
+        start.record()
+        for _ in range(5):
+            decode_linear(a, b, bias, weight_layout=layout)
+        end.record()
+        end.synchronize()
+        return start.elapsed_time(end)
+
+    got, strict = (decode_linear(x, weight, bias, weight_layout=layout, strict_fp32=s) for s in (False, True))
+    odd = torch.zeros(m, n, dtype=torch.bool, device="cuda")
+    odd[[3, 17, m - 1]] = True
+    odd[:, [2, n - 1]] = True
+    overflow = torch.zeros_like(odd)
+    overflow[20, 11] = True  # an infinity or a NaN, by the order of the sum
+    assert not torch.isfinite(strict[odd | overflow]).any() and not torch.isfinite(got[overflow]).any()
+    assert torch.isfinite(strict[~(odd | overflow)]).all()
+    assert torch.equal(got[odd].nan_to_num(nan=7.0, posinf=8.0, neginf=9.0), strict[odd].nan_to_num(nan=7.0, posinf=8.0, neginf=9.0))
+    same = ~odd
+    same[20], same[:, 11] = False, False
+    assert torch.equal(got[same], clean[same])  # finite outputs keep their bits
+    large = ~odd & ~overflow & ~same
+    assert rel_l2(got[large], strict[large]) <= 1e-6
+    assert times(torch.full_like(x, float("nan")), weight) <= 6 * times(torch.randn_like(x), torch.randn_like(weight))
