@@ -75,14 +75,18 @@ __device__ __forceinline__ void merge_stats(float& m_a, float& l_a, float& scale
 
 // ---- even split of a batch ---------------------------------------------------------------------------------------
 // Contexts differ from token to token, and only the device knows them.  The tiles of all (token, KV head) items stand
-// one behind the other, token-major, and CTA b of B takes tiles [b W / B, (b + 1) W / B) of the W there are.  An item
+// one behind the other, token-major, and CTA b of B takes tiles [b W / B, (b + 1) W / B) of the W there are (B: the CTAs of the
+// grid, or W, if there are fewer tiles than CTAs: the CTAs past W have no part in it).  An item
 // that lies inside one CTA is finished there; the others leave one partial result (max, sum, accumulator per head) per
 // CTA in scratch -- slot 2 b + 1 for the item that CTA b begins and does not end, slot 2 b for one begun before it --
 // and paged_decode_attention_merge_kernel adds them in CTA order.
 constexpr int kMergeThreads = 256;
 constexpr int kMaxTokensSplit = 16384;  // every CTA adds up the tiles of all tokens: longer batches have items enough
-// Shorter contexts stay on the grid of splits: finding the share and the second launch cost about 4 us, which the even split
-// only earns back on uneven or long ones.  us, contexts of every length up to the bound / all at the bound, even against
+// Shorter contexts stay on the grid of splits: finding the share and the second launch cost 1 .. 4 us, which the even split
+// only earns back on uneven or long ones.
+// Short contexts under a long bound cost no more: one token, 8 heads x 128, 512 positions, bound 8192 8.8 / 10.9, 16 tokens 11.9 / 12.5 (one
+// token of 2 heads x 64, 1024 positions 20.3 while CTAs without a share left zeros for the merge, which then had them all to add).
+// us, contexts of every length up to the bound / all at the bound, even against
 // splits: 16 tokens x 8 heads x 128, bound 512 13.8 / 13.3 against 12.3 / 14.9, 1024 15.9 / 19.4 against 15.9 / 18.1, 2048
 // 20.0 / 33.2 against 24.1 / 32.9; one token, 8192 13.9 / 16.8 against 14.9 / 24.8; FP32, 64 tokens x 4 heads, 2048 63 / 102 against 123 / 131.
 // Against the kernel before the even split, whose dead positions were read: 16 tokens, 8192 56 / 95 from 82 / 98; 64 tokens,
@@ -135,7 +139,10 @@ struct ItemCursor {  // a tile of an item
   }
 };
 
-// Sets `at` to this CTA's first tile and returns how many tiles it has; `batch_tiles` (in shared memory): tiles of the batch.
+// CTAs that have a share of `total` tiles; each of them has at least one.
+__device__ __forceinline__ int64_t share_ctas(int64_t total) { return total < gridDim.x ? total : gridDim.x; }
+
+// Sets `at` to this CTA's first tile and returns how many tiles it has, 0 for a CTA without a share; `batch_tiles` (in shared memory): tiles of the batch.
 // All threads call it.
 template <int U>
 __device__ __forceinline__ int64_t seek_share(const AttnArgs& a, ItemCursor& at, int64_t& batch_tiles, TokenCache& cache) {
@@ -163,8 +170,9 @@ __device__ __forceinline__ int64_t seek_share(const AttnArgs& a, ItemCursor& at,
 #pragma unroll
   for (int w = 0; w < kAttnWarps; ++w) total += warp_sums[w];
   if (threadIdx.x == 0) batch_tiles = total;
-  const int64_t w0 = total * blockIdx.x / gridDim.x, w1 = total * (blockIdx.x + 1) / gridDim.x;
-  if (w0 == w1) return 0;
+  const int64_t ctas = share_ctas(total);
+  if (blockIdx.x >= ctas) return 0;
+  const int64_t w0 = total * blockIdx.x / ctas, w1 = total * (blockIdx.x + 1) / ctas;
   int64_t before = 0;  // tiles of the tokens in front of the chunk
   for (int t0 = 0;; t0 += kAttnThreads) {
     const int64_t mine = t0 == 0 ? first : tiles_of(t0 + threadIdx.x);
@@ -207,9 +215,9 @@ __device__ __forceinline__ void finish_segment(const AttnArgs& a, const PeerOut&
   const bool ends = tiles_left == 0;  // of the item, behind this segment
   if (begins && !ends && threadIdx.x == 0) {
     // the CTA that holds the item's last tile: the tile's number in the batch is this CTA's last one + what is left
-    const int64_t last = total * (blockIdx.x + 1) / gridDim.x + tiles_left - 1;
+    const int64_t ctas = share_ctas(total), last = total * (blockIdx.x + 1) / ctas + tiles_left - 1;
     int* h = p.header + 4 * blockIdx.x;
-    h[0] = token, h[1] = kvh, h[2] = static_cast<int>(((last + 1) * gridDim.x - 1) / total);
+    h[0] = token, h[1] = kvh, h[2] = static_cast<int>(((last + 1) * ctas - 1) / total);
   }
   for (int i = threadIdx.x; i < G * D; i += kAttnThreads) {
     const int g = i / D, d = i - g * D;
@@ -227,15 +235,6 @@ __device__ __forceinline__ void finish_segment(const AttnArgs& a, const PeerOut&
     }
   }
   __syncthreads();
-}
-
-// A CTA without tiles may lie between two that share an item: its slot holds nothing.
-template <int G, int D>
-__device__ __forceinline__ void empty_share(const AttnArgs& a) {
-  const Partials<G, D> p(a.scratch, gridDim.x);
-  const int slot = 2 * blockIdx.x;
-  for (int i = threadIdx.x; i < G * D; i += kAttnThreads) p.acc[static_cast<size_t>(slot) * G * D + i] = 0.0f;
-  if (threadIdx.x < G) p.m[slot * G + threadIdx.x] = -INFINITY, p.l[slot * G + threadIdx.x] = 0.0f;
 }
 
 // Block b adds the partial results of the item that CTA b began and others went on with.  A thread owns four head dims and
@@ -345,10 +344,7 @@ paged_decode_attention_kernel(const T* q, const T* k_cache, const T* v_cache,
   if (even) {
     if (threadIdx.x == 0) Partials<G, D>(a.scratch, gridDim.x).header[4 * blockIdx.x] = -1;
     left_tiles = seek_share<kAttnThreads>(a, cur, batch_tiles, cache);
-    if (left_tiles == 0) {
-      empty_share<G, D>(a);
-      return;
-    }
+    if (left_tiles == 0) return;
   } else {
     cur.kvh = blockIdx.y, cur.token = blockIdx.z, cur.load<kAttnThreads>(a, nullptr);
   }
@@ -653,10 +649,7 @@ paged_decode_attention_tc_kernel(const T* q, const T* k_cache, const T* v_cache,
   if (even) {
     if (threadIdx.x == 0) Partials<G, D>(a.scratch, gridDim.x).header[4 * blockIdx.x] = -1;
     n_tiles = static_cast<int>(seek_share<Tile::kUnit>(a, cur, batch_tiles, cache));
-    if (n_tiles == 0) {
-      empty_share<G, D>(a);
-      return;
-    }
+    if (n_tiles == 0) return;
   } else {
     cur.kvh = blockIdx.y, cur.token = blockIdx.z, cur.load<Tile::kUnit>(a, nullptr);
     cur.tile = static_cast<int>(static_cast<int64_t>(cur.tiles) * split / splits);

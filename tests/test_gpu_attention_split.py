@@ -60,3 +60,20 @@ def test_attention_not_a_number_and_empty_contexts_show():
     got = paged_decode_attention(*(t.cuda() for t in (q, kc, vc, pos, table, seq)), page_size=16).cpu()
     assert torch.isnan(got[0, 4:]).all() and torch.isfinite(got[0, :4]).all()
     assert torch.isnan(got[1]).all() and torch.isfinite(got[2]).all()
+
+
+@pytest.mark.parametrize("heads,dim,tokens", [((8, 2), 64, 1), ((8, 2), 64, 4), ((8, 8), 128, 1), ((32, 8), 128, 2)])
+def test_short_contexts_under_a_long_bound(heads, dim, tokens):
+    """Few tiles on a grid sized for many: the CTAs without a share have no part in it, so a call takes about what the grid of
+    splits takes (it took up to 2.7 times as long while they left empty partial results to add up)."""
+    from cross_dsl_kernels_b200.ops import paged_decode_attention
+    from cross_dsl_kernels_b200.timing import graph_median_us
+    q, kc, vc, pos, table, seq = _paged(tokens, *heads, dim, 16, [8191] * tokens, torch.float16, seed=tokens)
+    pos = torch.full((tokens,), 1000)
+    want = oracle_attention.paged_decode_attention(q, kc, vc, pos, table, seq, page_size=16)
+    dev = [t.cuda() for t in (q, kc, vc, pos, table, seq)]
+    us = []
+    for hint in (0, 8192, 1024):  # even, even, splits
+        assert rel_l2(paged_decode_attention(*dev, page_size=16, context_hint=hint).cpu(), want) <= 1e-3
+        us.append(graph_median_us([lambda: paged_decode_attention(*dev, page_size=16, context_hint=hint)] * 8)["median_us"])
+    assert max(us[:2]) <= 1.5 * us[2], us
