@@ -275,6 +275,7 @@ PyObject* attention(PyObject*, PyObject* const* arg, Py_ssize_t n) {
   NEED(pos.size(0) == tokens && seq.size(0) == tokens);
   const double scale = arg[8] == Py_None ? std::pow(static_cast<double>(dim), -0.5) : PyFloat_AS_DOUBLE(arg[8]);
   NEED(std::isfinite(scale));
+  if (hint <= 0 && __builtin_mul_overflow(table.size(1), page, &hint)) hint = 0;  // no bound: that of a page table row
   at::Tensor out;
   int st;
   {

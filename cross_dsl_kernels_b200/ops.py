@@ -224,6 +224,9 @@ def paged_decode_attention(q, k_cache, v_cache, positions, page_table, sequence_
     :func:`rope_gqa_paged_kv_append` wrote (the token's own K/V included): FP32 softmax(scale * q.K) . V per head,
     GQA with q_heads / kv_heads in {1, 2, 4, 8}, head_dim in {64, 128, 256}.  Not part of upstream.
 
+    ``context_hint``: a bound on the context lengths, for the split of the work; any value gives the right result.  0: what a row
+    of the page table can hold.
+
     ``peer_out`` (multi-GPU; :meth:`cross_dsl_kernels_b200.peer.PeerMatrix.out_for`): the result goes to columns
     [col0, col0 + q_heads * head_dim) of every rank's copy of a [tokens, all heads * head_dim] matrix instead of a
     fresh tensor, and the call returns None; readers wait for the arena's flag barrier."""
@@ -265,12 +268,15 @@ def paged_decode_attention(q, k_cache, v_cache, positions, page_table, sequence_
             _need(peer_out.ld >= peer_out.col0 + q_heads * head_dim, "peer_out is narrower than col0 + q_heads * head_dim")
             out, dst = None, peer_out
         # partial results of (token, KV head) pairs that several CTAs share: a fresh block per call, as in decode_linear
-        need = lib.xdk_paged_decode_attention_scratch_bytes(tokens, q_heads, kv_heads, head_dim, int(context_hint), code)
+        hint = int(context_hint)
+        if hint <= 0:  # no bound: that of a page table row
+            hint = min(page_table.shape[1] * page_size, 2 ** 62)
+        need = lib.xdk_paged_decode_attention_scratch_bytes(tokens, q_heads, kv_heads, head_dim, hint, code)
         scratch = torch.empty(need, device=q.device, dtype=torch.uint8) if need else None
         status = lib.xdk_paged_decode_attention_ws(
             q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), positions.data_ptr(), page_table.data_ptr(),
             sequence_ids.data_ptr(), ctypes.byref(dst), tokens, q_heads, kv_heads, head_dim, page_table.shape[1], page_size,
-            int(layout == "HND"), scale, int(context_hint), code, scratch.data_ptr() if need else None, need,
+            int(layout == "HND"), scale, hint, code, scratch.data_ptr() if need else None, need,
             _flags(dependent_launch), _native.stream_ptr(q.device))
     _native.check(status, "xdk_paged_decode_attention")
     return out

@@ -260,7 +260,7 @@ XDK_API int xdk_w4a16_v2(const void* x, const uint8_t* packed, const void* scale
  *   K/V are in the cache already), G = q_heads / kv_heads in {1, 2, 4, 8}, head_dim in {64, 128, 256}; q and out
  *   [tokens, q_heads, head_dim] contiguous; caches, positions, page_table, sequence_ids and the address
  *   translation exactly as in xdk_rope_kv_append.  FP32 scores, softmax and accumulation.  context_hint: the longest
- *   context the caller expects (bounds how finely the context is split across CTAs; <= 0: long).  One launch, no
+ *   context the caller expects (bounds how finely the context is split across CTAs; <= 0: what a page table row holds).  One launch, no
  *   scratch: the slices of a (token, KV head) are merged through distributed shared memory in a fixed order.
  * xdk_swiglu: out[r][j] = silu(upgate[r][width + j]) * upgate[r][j] for j < width -- columns [0, width) of the fused
  *   projection are "up", [width, 2 width) "gate"; in_ld / out_ld: elements between rows.

@@ -2,6 +2,8 @@
 
 from __future__ import annotations
 
+import ctypes
+
 import pytest
 import torch
 
@@ -77,3 +79,26 @@ def test_short_contexts_under_a_long_bound(heads, dim, tokens):
         assert rel_l2(paged_decode_attention(*dev, page_size=16, context_hint=hint).cpu(), want) <= 1e-3
         us.append(graph_median_us([lambda: paged_decode_attention(*dev, page_size=16, context_hint=hint)] * 8)["median_us"])
     assert max(us[:2]) <= 1.5 * us[2], us
+
+
+@pytest.mark.parametrize("page,pages", [(16, 64), (5, 100), (64, 20), (16, 200), (1, 1535), (1, 1537)])
+def test_no_bound_is_that_of_the_page_table(page, pages):
+    """A call without a context_hint is the call with what a row of the page table can hold: the same plan, the same bits."""
+    from cross_dsl_kernels_b200 import _native
+    from cross_dsl_kernels_b200.ops import paged_decode_attention
+    tokens, heads, dim = 3, (6, 3), 64
+    q, kc, vc, pos, table, seq = _paged(tokens, *heads, dim, page, [page * pages - 1, page * pages // 2, 0], torch.float32, seed=pages)
+    dev = [t.cuda() for t in (q, kc, vc, pos, table, seq)]
+    want = paged_decode_attention(*dev, page_size=page, context_hint=page * pages)
+    for hint in (0, -1, -2 ** 63):
+        assert torch.equal(paged_decode_attention(*dev, page_size=page, context_hint=hint), want)
+    out = torch.empty_like(dev[0])  # a C caller sizes its scratch for no bound, and passes none
+    size = _native.lib().xdk_paged_decode_attention_scratch_bytes(tokens, *heads, dim, 0, _native.XDK_F32)
+    scratch = torch.empty(size, dtype=torch.uint8, device="cuda")
+    dst = _native.PeerOutStruct()
+    dst.ptr[0], dst.world, dst.ld, dst.col0 = out.data_ptr(), 1, heads[0] * dim, 0
+    status = _native.lib().xdk_paged_decode_attention_ws(
+        *(t.data_ptr() for t in dev), ctypes.byref(dst), tokens, *heads, dim, pages, page, 0, dim ** -0.5, 0, _native.XDK_F32, scratch.data_ptr(), size,
+        0, _native.stream_ptr(out.device))
+    _native.check(status, "attention")
+    assert torch.equal(out, want)
