@@ -9,9 +9,11 @@ from __future__ import annotations
 import ctypes
 import functools
 import pathlib
+import re
+import sysconfig
+import warnings
 
 LIB_PATH = pathlib.Path(__file__).resolve().parent / "libxdk_b200.so"
-HOST_PATH = LIB_PATH.with_name("_host.so")
 
 XDK_F32, XDK_BF16, XDK_F16 = 0, 1, 2
 XDK_STRICT_FP32, XDK_DEPENDENT_LAUNCH = 1, 2  # flags of the *_v2 entry points
@@ -91,19 +93,36 @@ def lib() -> ctypes.CDLL:
     return handle
 
 
+def host_path() -> pathlib.Path:
+    """Where the native half of the ops for this torch and this interpreter lies.  It is compiled against the C++ headers of the
+    one and the C API of the other, so its name carries both: what was built for others is never loaded."""
+    import torch
+
+    built_for = re.sub(r"[^0-9A-Za-z]+", "_", f"torch{torch.__version__}_{sysconfig.get_config_var('SOABI')}")
+    return LIB_PATH.with_name(f"_host.{built_for}.so")
+
+
+class _Declines:
+    """In the place of the native half where it was not built: the Python functions take every call."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
 @functools.lru_cache(maxsize=1)
 def host():
     """The native half of the ops (csrc/host.cpp): each function launches an ordinary call, or returns None."""
     import importlib.machinery
     import importlib.util
 
-    import torch  # noqa: F401  (its libraries first: the extension links against them)
-
-    if not HOST_PATH.exists():
-        raise NativeLibraryError(f"{HOST_PATH} is not built; run `python -m cross_dsl_kernels_b200.build`")
     lib()
-    loader = importlib.machinery.ExtensionFileLoader("_host", str(HOST_PATH))
-    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_host", str(HOST_PATH), loader=loader))
+    path = host_path()  # imports torch, whose libraries the extension links against
+    if not path.exists():
+        warnings.warn(f"{path} is not built for this torch and Python: eager ops are checked in Python, at several times the cost "
+                      "of a call; run `python -m cross_dsl_kernels_b200.build`", RuntimeWarning, stacklevel=3)
+        return _Declines()
+    loader = importlib.machinery.ExtensionFileLoader("_host", str(path))
+    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_host", str(path), loader=loader))
     loader.exec_module(module)
     module.set_check(check)
     return module

@@ -43,6 +43,32 @@ def test_it_declines_what_is_not_on_a_gpu_and_odd_argument_lists():
         assert getattr(host, name)(*[None] * 20) is None
 
 
+def test_it_is_built_for_one_torch_and_one_python_and_may_be_missing(monkeypatch):
+    """Its name carries what it was compiled against; where it was not built, every call goes to the Python functions."""
+    from cross_dsl_kernels_b200 import build
+    ours = _native.host_path()
+    assert ours.exists() and build.host_target() == ours and not build.needs_build()
+    monkeypatch.setattr(torch, "__version__", "99.0+other")
+    assert _native.host_path() != ours and build.needs_build()
+    _native.host.cache_clear()
+    try:
+        with pytest.warns(RuntimeWarning, match="not built"):
+            host = _native.host()
+        assert all(getattr(host, name)(1, 2) is None for name in NAMES)
+        with pytest.raises(ValueError, match="CUDA"):
+            ops.swiglu(torch.zeros(2, 8))
+    finally:
+        _native.host.cache_clear()
+    assert f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}" in build._host_command(ours)
+
+
+def test_the_library_builds_without_a_torch_that_has_cuda(monkeypatch):
+    import torch.utils.cpp_extension
+    from cross_dsl_kernels_b200 import build
+    monkeypatch.setattr(torch.utils.cpp_extension, "library_paths", lambda *a, **k: [])
+    assert build.host_target() is None and not build.needs_build()
+
+
 @pytest.mark.gpu
 def test_ordinary_calls_give_the_same_bits(monkeypatch):
     g = torch.Generator(device="cuda").manual_seed(0)
