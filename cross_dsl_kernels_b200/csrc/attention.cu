@@ -52,17 +52,13 @@ struct AttnArgs {
   float* scratch;  // even split of the batch's tiles over the grid, partial results here; nullptr: grid = (splits, heads, tokens)
 };
 
-// 16 bytes, or zeros and no access (bytes = 0) for a dead position.  (Dead positions used to read row 0 of the cache: with
+// 16 bytes of a row, or zeros and no access for a dead position (row < 0).  (Dead positions used to read row 0 of the cache: with
 // contexts of every length that was megabytes from one line, and its L2 slice set the time -- 64 contexts of 1 .. 2048 took
 // longer than 64 of 2048.)
-__device__ __forceinline__ void cp_async16_or_zero(void* dst_smem, const unsigned char* src, int bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst_smem)), "l"(src), "r"(bytes) : "memory");
-}
 template <typename T>
-__device__ __forceinline__ void cp_async16_row(void* dst_smem, const T* cache, int64_t row, int at) {  // row < 0: dead
-  cp_async16_or_zero(dst_smem, reinterpret_cast<const unsigned char*>(cache + (row < 0 ? 0 : row)) + at, row < 0 ? 0 : 16);
+__device__ __forceinline__ void cp_async16_row(void* dst_smem, const T* cache, int64_t row, int at) {
+  cp_async16_or_zero(dst_smem, reinterpret_cast<const unsigned char*>(cache + (row < 0 ? 0 : row)) + at, row >= 0);
 }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Merges partial (m, l, acc) `b` into `a` (online softmax): both cover disjoint position sets.
 __device__ __forceinline__ void merge_stats(float& m_a, float& l_a, float& scale_a, float& scale_b, float m_b, float l_b) {
@@ -97,19 +93,22 @@ constexpr int kMinEvenContext = 1536;
 // roundings up, inside 64 bits.
 constexpr int64_t kMaxContextHint = 1LL << 38;
 
+// 32-bit words of the parts of a grid's scratch, in the order they lie there
+struct PartialWords {
+  size_t acc, stat, header;  // [2 ctas][g * d] accumulators, [2 ctas][g] twice (m, l), [ctas][4]
+  __host__ __device__ constexpr PartialWords(size_t ctas, size_t g, size_t d) : acc(2 * ctas * g * d), stat(2 * ctas * g), header(4 * ctas) {}
+  __host__ __device__ constexpr size_t all() const { return acc + 2 * stat + header; }
+};
 template <int G, int D>
 struct Partials {  // scratch of a grid of `ctas`
   float* acc;      // [2 ctas][G * D]
   float* m;        // [2 ctas][G]
   float* l;        // [2 ctas][G]
   int* header;     // [ctas][4]: token, KV head, CTA that ends the item that CTA b begins; token < 0: none
-  __host__ __device__ Partials(float* base, int ctas) {
-    acc = base;
-    m = acc + static_cast<size_t>(2) * ctas * G * D;
-    l = m + static_cast<size_t>(2) * ctas * G;
-    header = reinterpret_cast<int*>(l + static_cast<size_t>(2) * ctas * G);
+  __device__ Partials(float* base, unsigned ctas) {
+    const PartialWords words(ctas, G, D);
+    acc = base, m = acc + words.acc, l = m + words.stat, header = reinterpret_cast<int*>(l + words.stat);
   }
-  static size_t bytes(int ctas) { return (static_cast<size_t>(2) * ctas * (G * D + 2 * G) + static_cast<size_t>(4) * ctas) * 4; }
 };
 
 // Context length and sequence of the batch's first tokens, in shared memory: a step to the next item would otherwise cost two
@@ -712,9 +711,9 @@ paged_decode_attention_tc_kernel(const T* q, const T* k_cache, const T* v_cache,
     for (int i = 0; i < PIECES; ++i) {
       const int c = i * 32 + lane, r = c / PIECES, p = c - r * PIECES;
       const unsigned char* src = reinterpret_cast<const unsigned char*>(rows[warp][r]) + p * 16;
-      const int bytes = r < live_end ? 16 : 0;
-      cp_async16_or_zero(ktile + r * kPitch + p * 16, src, bytes);
-      cp_async16_or_zero(vtile + r * kPitch + p * 16, src + v_from_k, bytes);
+      const bool live = r < live_end;
+      cp_async16_or_zero(ktile + r * kPitch + p * 16, src, live);
+      cp_async16_or_zero(vtile + r * kPitch + p * 16, src + v_from_k, live);
     }
     const int token = cur.token, kvh = cur.kvh, tiles_left = cur.tiles - 1 - cur.tile;
     if (fresh) {
@@ -970,7 +969,7 @@ extern "C" size_t xdk_paged_decode_attention_scratch_bytes(int64_t tokens, int64
   if (head_dim != 64 && head_dim != 128 && head_dim != 256) return 0;
   const int g = static_cast<int>(q_heads / kv_heads);
   const int ctas = even_grid(tokens, kv_heads, head_dim, context_hint, dtype == XDK_F32 ? 4 : 2, g);
-  return static_cast<size_t>(ctas) * (2 * (g * static_cast<size_t>(head_dim) + 2 * g) + 4) * 4;
+  return PartialWords(ctas, g, head_dim).all() * 4;
 }
 
 extern "C" int xdk_paged_decode_attention_ws(const void* q, const void* k_cache, const void* v_cache, const int64_t* positions,

@@ -57,13 +57,6 @@ struct MmaArgs {
   int block0;  // first block of 16 rows of this launch
 };
 
-__device__ __forceinline__ void cp_async16_or_zero(void* dst, const void* src, bool live) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(live ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
 struct Split {
   uint32_t hi, lo, lead;  // lead: the factor of the leading product, hi but for what does not split
 };

@@ -1279,20 +1279,18 @@ w4a16_rx_kernel(W4Args a, RxPlan plan, const __grid_constant__ CUtensorMap wmap)
   if (plan.ranks > 1) cg::this_cluster().barrier_wait();
 
   bool ok = true;
-  const size_t out_at = static_cast<size_t>(q * 2) * a.out.ld + a.out.col0 + g0 * 16 + col_lo;
+  const size_t out_at = static_cast<size_t>(q * 2) * a.n + g0 * 16 + col_lo;  // plain outputs only: strided ones go elsewhere
   auto store = [&](int pass, const float4 (&sum)[MR]) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int col = (g0 + pass) * 16 + h * 8 + col_lo;
       if (col >= a.n) continue;
       const float bv = a.bias ? __half2float(a.bias[col]) : 0.0f;
-      for (int p = 0; p < a.out.world; ++p) {
-        __half* dst = static_cast<__half*>(a.out.ptr[p]) + out_at + pass * 16 + h * 8;
+      __half* dst = a.y + out_at + pass * 16 + h * 8;
 #pragma unroll
-        for (int r = 0; r < MR; ++r) {
-          if (r * 8 + q * 2 < a.m) dst[r * 8 * a.out.ld] = __float2half_rn((h ? sum[r].z : sum[r].x) + bv);
-          if (r * 8 + q * 2 + 1 < a.m) dst[(r * 8 + 1) * a.out.ld] = __float2half_rn((h ? sum[r].w : sum[r].y) + bv);
-        }
+      for (int r = 0; r < MR; ++r) {
+        if (r * 8 + q * 2 < a.m) dst[static_cast<size_t>(r) * 8 * a.n] = __float2half_rn((h ? sum[r].z : sum[r].x) + bv);
+        if (r * 8 + q * 2 + 1 < a.m) dst[static_cast<size_t>(r * 8 + 1) * a.n] = __float2half_rn((h ? sum[r].w : sum[r].y) + bv);
       }
     }
   };
