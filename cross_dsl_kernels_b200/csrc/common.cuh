@@ -143,14 +143,6 @@ __device__ __forceinline__ U4 ld_ordered16(const void* p) {
   asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ U4 ld_ordered16_if(const void* p, bool live) {  // zeros and no access where not live; no branch
-  U4 v;
-  asm volatile(
-      "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
-      "@q ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}"
-      : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w) : "l"(p), "r"(static_cast<unsigned>(live)) : "memory");
-  return v;
-}
 __device__ __forceinline__ U4 ld_ordered_stream16(const void* p) {  // each byte is used once: not kept in L1
   U4 v;
   asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"

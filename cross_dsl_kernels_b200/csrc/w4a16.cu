@@ -23,6 +23,7 @@
 #include <stdlib.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 #include "umma.cuh"
@@ -1046,27 +1047,32 @@ w4a16_mma_kernel(W4Args a, int col_groups) {
   fetch(buf0, cta_col0, 0);  // the first batch's weights go out before x is staged
   pdl_wait();                // x may be the preceding kernel's output; the weights are not
 
+  // x into shared memory: 16 bytes per thread and load, eight loads in flight, then four, two and one for the rest (K % 1024 == 0: the
+  // same for all threads of a warp)
   const int units = a.k / 8, x_units = a.m * units;
-  constexpr int kXFlight = 8;  // ordered loads in flight per thread
   const uint32_t per_unit = 0xffffffffu / units + 1;  // i / units = the high word of i * per_unit, for i * units below 2^32
-  for (int i0 = threadIdx.x; i0 < x_units; i0 += kXFlight * kThreads) {
-    U4 v[kXFlight];
+  int at = threadIdx.x;
+  auto stage = [&](auto flight) {
+    constexpr int F = decltype(flight)::value;
+    U4 v[F];
 #pragma unroll
-    for (int j = 0; j < kXFlight; ++j)
-      v[j] = ld_ordered16_if(a.x + static_cast<size_t>(i0 + j * kThreads) * 8, i0 + j * kThreads < x_units);
+    for (int j = 0; j < F; ++j) v[j] = ld_ordered16(a.x + static_cast<size_t>(at + j * kThreads) * 8);
 #pragma unroll
-    for (int j = 0; j < kXFlight; ++j) {
-      const int i = i0 + j * kThreads, r = static_cast<int>(__umulhi(i, per_unit));
-      if (i < x_units) {
-        U4 o;  // k 0..7 -> 0,4,1,5,2,6,3,7: the pairs the unpack produces
-        o.x = __byte_perm(v[j].x, v[j].z, 0x5410);
-        o.y = __byte_perm(v[j].x, v[j].z, 0x7632);
-        o.z = __byte_perm(v[j].y, v[j].w, 0x5410);
-        o.w = __byte_perm(v[j].y, v[j].w, 0x7632);
-        *reinterpret_cast<U4*>(xs + (i + r) * 16) = o;  // 16 bytes of pad behind every row
-      }
+    for (int j = 0; j < F; ++j) {
+      const int i = at + j * kThreads, r = static_cast<int>(__umulhi(i, per_unit));
+      U4 o;  // k 0..7 -> 0,4,1,5,2,6,3,7: the pairs the unpack produces
+      o.x = __byte_perm(v[j].x, v[j].z, 0x5410);
+      o.y = __byte_perm(v[j].x, v[j].z, 0x7632);
+      o.z = __byte_perm(v[j].y, v[j].w, 0x5410);
+      o.w = __byte_perm(v[j].y, v[j].w, 0x7632);
+      *reinterpret_cast<U4*>(xs + (i + r) * 16) = o;  // 16 bytes of pad behind every row
     }
-  }
+    at += F * kThreads;
+  };
+  while (at + 7 * kThreads < x_units) stage(std::integral_constant<int, 8>{});
+  if (at + 3 * kThreads < x_units) stage(std::integral_constant<int, 4>{});
+  if (at + kThreads < x_units) stage(std::integral_constant<int, 2>{});
+  if (at < x_units) stage(std::integral_constant<int, 1>{});
   __syncthreads();
   // this lane's B fragments: row n of x; lanes past M read row 0 and feed output rows that are never stored
   const unsigned char* xrow = xs + static_cast<size_t>(n < a.m ? n : 0) * pitch;
