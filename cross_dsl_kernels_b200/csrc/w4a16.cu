@@ -15,7 +15,7 @@
 //     tcgen05 kind::f16 with the dequantised weights in tensor memory (w4a16_umma_kernel).
 //   * the other M >= 3, K % 128 == 0: the same MMAs with x kept in registers and K shared by the warps of a CTA or the
 //     CTAs of a cluster (w4a16_rx_kernel).
-//   * the rest: a TMA-fed mma.sync stream kernel (K > 32768), a SIMT kernel (lanes stride over the packed row,
+//   * the rest: a TMA-fed mma.sync stream kernel (short K of M >= 9, K > 32768), a SIMT kernel (lanes stride over the packed row,
 //     mixed-precision FMAs, warp shuffle per column) and a generic kernel for any K.
 // The k order inside an MMA fragment is free as long as both operands use the same order, so x is stored in shared
 // memory pre-permuted to the order the unpack produces and no weight ever moves between lanes.
@@ -187,7 +187,7 @@ __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1
 __device__ __forceinline__ int xunit(int unit, int row) { return unit ^ ((((unit >> 3) & 1) << 1) | (row & 1)); }
 
 // ------------------------------------------------------------------------------------------------
-// Streaming tensor-core path (M >= 3, K % 128 == 0, K too long for the paths below).
+// Streaming tensor-core path (M >= 3, K % 128 == 0: a short K of M >= 9, and K too long for the paths below).
 //
 // One persistent CTA per SM.  The N/8 column blocks are dealt out evenly to clusters of S CTAs
 // (S = split-K factor, 1/2/4); inside a cluster CTA r takes the K chunks r, r+S, ... of 1024 k, and
@@ -1428,8 +1428,9 @@ int rx_resident_clusters(int ranks) {  // the same for every variant: one CTA pe
   return n;
 }
 
+// XDK_ERR_LIMIT: K > 32768, or more columns than the resident clusters take in one wave when `one_wave` asks for it.
 template <int MR>
-int launch_rx(const W4Args& a, bool dependent, cudaStream_t stream) {
+int launch_rx(const W4Args& a, bool dependent, bool one_wave, cudaStream_t stream) {
   RxPlan p = {};
   cudaError_t err = cudaFuncSetAttribute(w4a16_rx_kernel<MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRxSmem);
   if (err != cudaSuccess) return note_launch(err);
@@ -1452,6 +1453,7 @@ int launch_rx(const W4Args& a, bool dependent, cudaStream_t stream) {
     if (clusters < 1) return XDK_ERR_LIMIT;
     clusters = min(clusters, p.groups);
     p.total_sets = max(clusters, (p.groups + kRxMaxPasses - 1) / kRxMaxPasses);
+    if (one_wave && p.total_sets > clusters) return XDK_ERR_LIMIT;
   }
   passes = (p.groups + p.total_sets - 1) / p.total_sets;
   p.parked = p.ranks > 1 ? (passes + p.ranks - 1) / p.ranks : 0;
@@ -1544,35 +1546,54 @@ extern "C" int xdk_w4a16_peer(const void* x, const uint8_t* packed, const void* 
   //  * M <= 2, K a multiple of 1024, and M <= 8 while x leaves room for two CTAs per SM: the direct-load mma.sync kernel
   //    (N = 4096 6.0 / 6.5 / 7.3 at M = 1 / 4 / 8, N = 14336 14.7 / 15.7 / 16.4; the kernel that keeps x in registers 7.6 /
   //    7.9 / 8.5 and 16.4 / 17.2 / 17.7; the SIMT kernel 16.3 at M = 1, N = 14336).
-  //  * M >= 9 where the tcgen05 kernel's CTAs walk whole strips, three or four 32-column units wide, or two of a short K:
-  //    the tcgen05 kernel (M = 16: N = 14336 17.6 against 20.8, N = 16384 17.7 / 21.2, N = 8192 13.9 / 14.5), and every
-  //    strided or multi-rank output.
-  //  * every other M >= 3: the kernel that keeps x in registers.  M = 16: one unit a CTA, i.e. K split over the lane
-  //    quarters (N = 2048 8.0 against 10.9, K = 14336, N = 4096 22.6 / 34.0, K = 11008 19.6 / 30.5), a strip and a narrow rest
-  //    (N = 24576 26.0 / 27.2), shapes the tcgen05 kernel declines (K = 2304, N = 8192 11.8 / 15.5); M = 8: x too large for two
-  //    CTAs (K = 14336, N = 4096 18.9 / 27.9, K = 7168, N = 20480 29.6 / 39.9), K = 2304, N = 8192 9.8 / 14.1.
+  //    A larger x too where every SM has one group of columns at most anyway and most have one (M = 8, K = 7168, N = 2048
+  //    8.6 / 9.3, N = 2368 8.7 / 9.5, but N = 1024 8.1 / 7.4; K = 9216, N = 2048 10.6 / 10.2).
+  //  * M >= 9, figures for 16, the tcgen05 kernel / the one that keeps x in registers, by the 32-column units of the former's
+  //    busiest CTA.  K up to 4096: the former where its CTAs walk whole strips of three or four units, or two (N = 14336 17.6 / 20.8,
+  //    N = 18944 17.9 / 22.0, N = 8192 13.9 / 14.5; but one unit, K split over the lane quarters, N = 2048 10.7 / 7.7, a strip and a
+  //    narrow rest N = 23680 24.5 / 23.8, N = 33152 30.4 / 29.5; from K = 2048 to 4096 the former there too, K = 3072, N = 33112 24.0 / 24.8 at M = 9).
+  //    K up to 12288: the former from two units on (K = 5120, N = 9472 15.6 / 18.7, N = 23680 28.3 / 32.5; K = 10240, N = 9472 24.7 / 29.2,
+  //    N = 33112 64 / 77; K = 12288, N = 18904 41.1 / 49.5; K = 8192, where the latter's warps are all busy, either way: N = 9472 22.1 / 23.4,
+  //    N = 23680 44 / 40, N = 37888 56 / 58), and for a wide single one (N = 4696, K = 5120 12.4 / 13.0, 10240 18.8 / 20.8, but 8192 17.0 / 16.2;
+  //    N = 3584, K = 5120 12.3 / 12.3, 10240 18.4 / 17.0, N = 2400 18.1 / 14.8).
+  //    Longer K: the latter (K = 14336, N = 4096 34.0 / 22.6, N = 14208 66 / 49, N = 33152 133 / 103; K = 20480, N = 9432 75 / 44), as long as the
+  //    resident clusters take all columns in one wave (K = 14336, N = 37888 150 / 205).
+  //    Shapes the tcgen05 kernel declines: the latter (K = 2304, N = 8192 15.5 / 11.8 with the stream kernel, K = 896, N = 23640 11.9 / 11.6),
+  //    but for a short K on a middling width (K = 384, N = 9432 4.5 / 5.0, K = 896 6.4 / 7.6, N = 4096 4.7 / 5.2).
+  //    Every strided or multi-rank output: the tcgen05 kernel.
+  //  * 3 <= M <= 8 otherwise: the kernel that keeps x in registers.  M = 8: x too large for two CTAs (K = 14336, N = 4096 18.9, tcgen05
+  //    27.9, K = 7168, N = 20480 29.6 / 39.9), K = 2304, N = 8192 9.8 / 14.1.  But the tcgen05 kernel for strips of four units of a K between 8192
+  //    and 12288 (M = 8, K = 10240, N = 18904 34.1 / 40.4), and the direct-load one, x permitting, for more columns than one wave takes (M = 3,
+  //    K = 20480, N = 28672 135 / 166).
   // XDK_W4A16_MMA=0 and XDK_W4A16_UMMA=0 / 1 take the first kernel out, and the second out or in wherever it can run
   // (comparison runs).
   static const bool mma_env = !(getenv("XDK_W4A16_MMA") && getenv("XDK_W4A16_MMA")[0] == '0');
   static const int umma_env = getenv("XDK_W4A16_UMMA") ? (getenv("XDK_W4A16_UMMA")[0] == '1' ? 1 : 0) : -1;
   const size_t x_bytes = static_cast<size_t>(m) * (static_cast<size_t>(k) * 2 + 16);
-  if (mma_env && plain && vec_ok && k % 1024 == 0 && (m <= 2 ? x_bytes <= 160 * 1024 : m <= 8 && x_bytes <= 104 * 1024))
-  {
+  const int64_t groups = (n + 15) / 16, sms = sm_count();
+  const bool one_each = groups <= sms && (groups * 8 > sms * 7 || (groups * 4 > sms * 3 && k <= 8192));  // group of 16 columns on most SMs
+  if (mma_env && plain && vec_ok && k % 1024 == 0 &&
+      (m <= 2 || (m <= 8 && one_each) ? x_bytes <= 160 * 1024 : m <= 8 && x_bytes <= 104 * 1024)) {
     // Three CTAs per SM where that saves a pass over the column groups, or K is short (us with two / three, M = 1: K = 4096,
     // N = 6144 9.3 / 7.7, N = 20480 17.6 / 16.0, N = 28672 23.3 / 22.8, N = 8192 -- two passes either way -- 9.7 / 10.6; K = 2048,
     // N = 8192 6.6 / 6.3, N = 28672 16.1 / 13.8; M = 4 alike).  A larger x leaves the L1 cache too little for the scales.
-    const int64_t groups = (n + 15) / 16, two = 2LL * sm_count(), three = 3LL * sm_count();
+    const int64_t two = 2 * sms, three = 3 * sms;
     if (x_bytes <= 40 * 1024 && k <= 4096 && groups > two && (k <= 2048 || (groups + three - 1) / three < (groups + two - 1) / two))
       return launch_mma<2, 3>(a, dependent, s);
     return launch_mma<4, 2>(a, dependent, s);
   }
   const bool umma_ok = vec_ok && k % 256 == 0 && group_size >= 64 && a.groups <= 256 && a.groups % 8 == 0 && aligned16(scales);
-  const int64_t units = ((n + 31) / 32 + sm_count() - 1) / sm_count();  // 32-column units of the tcgen05 kernel's busiest CTA
-  const bool whole = units % 4 == 0 || units == 3 || (units == 2 && k < 8192) || (units > 4 && k > 4096);
-  const bool umma_first = !plain || umma_env == 1 || (m > 8 && whole && umma_env != 0);
-  if (plain && vec_ok && k % 128 == 0 && m >= 3 && !(umma_ok && umma_first)) {
-    const int st = m > 8 ? launch_rx<2>(a, dependent, s) : launch_rx<1>(a, dependent, s);
-    if (st != XDK_ERR_LIMIT) return st;  // K > 32768: the kernels below
+  const int64_t units = ((n + 31) / 32 + sms - 1) / sms;  // 32-column units of the tcgen05 kernel's busiest CTA
+  const bool whole = k <= 4096    ? units % 4 == 0 || units == 2 || units == 3 || (units > 4 && k >= 2048 && k < 4096)
+                     : k <= 12288 ? units >= 2 || (k != 8192 && n >= (k > 10240 ? 4097 : 4096))
+                                  : false;
+  const bool umma_first = !plain || umma_env == 1 || (umma_env != 0 && (m > 8 ? whole : units % 4 == 0 && k > 8192 && k <= 12288));
+  const bool stream_first = m > 8 && k < 1024 && n >= (k <= 128 ? 1 : (k <= 384 ? 2048 : 3072)) && n <= 4 * 32 * sms;
+  if (plain && vec_ok && k % 128 == 0 && m >= 3 && !(umma_ok && umma_first) && !stream_first) {
+    const bool umma_next = umma_ok && umma_env != 0;
+    const int st = m > 8 ? launch_rx<2>(a, dependent, umma_next, s) : launch_rx<1>(a, dependent, umma_next, s);
+    if (st != XDK_ERR_LIMIT) return st;  // the kernels below
+    if (mma_env && m <= 8 && k % 1024 == 0 && x_bytes <= 160 * 1024) return launch_mma<4, 2>(a, dependent, s);
   }
   if (umma_ok && (!plain || (umma_env != 0 && (m >= 3 || (m == 2 && k * n >= (32LL << 20)))))) {
     const int st = launch_umma(a, dependent, s);

@@ -58,3 +58,25 @@ def test_w4a16_large_scales_on_a_last_half_slice(m, k):
     codes = qz.unpack_int4(packed, k).double()
     want = x.double() @ (codes * scales.double().repeat_interleave(128, dim=1)[:, :k]).half().double().t()
     assert torch.equal(got, want.half())
+
+
+@pytest.mark.parametrize("k,n", [
+    (128, 1000), (384, 2048), (896, 4696),  # short K of many rows: the stream kernel
+    (7168, 2368),   # one column group per SM: the direct-load kernel up to M = 8
+    (10240, 4096), (10240, 18904), (12288, 9432),  # the tcgen05 kernel from M = 9, and for whole strips below
+    (14336, 14208),  # the kernel with x in registers
+    (14336, 37888), (20480, 28672),  # more columns than its clusters take in one wave
+])
+def test_w4a16_on_both_sides_of_the_dispatch(k, n):
+    """As above, on the GPU: the sums of small integers are exact in FP32, whichever kernel has the shape."""
+    from cross_dsl_kernels_b200.w4a16 import w4a16_linear
+    g = torch.Generator(device="cuda").manual_seed(k + n)
+    low, high = (torch.randint(7, 10, (n, k // 2), generator=g, device="cuda", dtype=torch.uint8) for _ in range(2))
+    packed = low + 16 * high  # codes of -1, 0 and 1
+    scales = torch.full((n, k // 128), 0.5, device="cuda").half()
+    codes = torch.stack((packed & 15, packed >> 4), dim=2).flatten(1).float() - 8
+    for m in (3, 8, 9, 16):
+        x = (torch.randint(0, 16, (m, k), generator=g, device="cuda") == 0).half() * torch.randint(-1, 2, (m, k), generator=g, device="cuda").half()
+        want = (x.float() @ codes.t() * 0.5).half()
+        for dependent in (False, True):
+            assert torch.equal(w4a16_linear(x, packed, scales, group_size=128, dependent_launch=dependent), want)
