@@ -114,17 +114,28 @@ rmsnorm_generic_kernel(const T* x, const T* residual, const T* __restrict__ weig
   pdl_launch_dependents();
   pdl_wait();
   const size_t base = static_cast<size_t>(blockIdx.x) * hidden;
+  // Eight elements at a time, their loads together: a load may not pass a store that could write what it reads.
+  const T *xr = x + base, *rr = residual + base;
+  auto each = [&](auto use) {  // use(i, FP32 sum of element i) for this thread's elements
+    int64_t i = threadIdx.x;
+    for (; i + 7 * 256 < hidden; i += 8 * 256) {
+      T a[8], b[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) a[j] = xr[i + j * 256], b[j] = rr[i + j * 256];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) use(i + j * 256, __fadd_rn(Elem<T>::to_f32(a[j]), Elem<T>::to_f32(b[j])));
+    }
+    for (; i < hidden; i += 256) use(i, __fadd_rn(Elem<T>::to_f32(xr[i]), Elem<T>::to_f32(rr[i])));
+  };
   float sum_sq = 0.0f;
-  for (int64_t i = threadIdx.x; i < hidden; i += 256) {
-    const float r = __fadd_rn(Elem<T>::to_f32(x[base + i]), Elem<T>::to_f32(residual[base + i]));
+  each([&](int64_t i, float r) {
     residual_out[base + i] = Elem<T>::from_f32(r);
     sum_sq = fmaf(r, r, sum_sq);
-  }
+  });
   const float scale = inv_rms(block_sum<256>(sum_sq, scratch), hidden_f, eps);
-  for (int64_t i = threadIdx.x; i < hidden; i += 256) {
-    const float r = __fadd_rn(Elem<T>::to_f32(x[base + i]), Elem<T>::to_f32(residual[base + i]));
+  each([&](int64_t i, float r) {
     y[base + i] = Elem<T>::from_f32(__fmul_rn(__fmul_rn(r, scale), Elem<T>::to_f32(weight[i])));
-  }
+  });
 }
 
 template <typename T, int THREADS, int VPT>
