@@ -93,21 +93,21 @@ constexpr int kMinEvenContext = 1536;
 // roundings up, inside 64 bits.
 constexpr int64_t kMaxContextHint = 1LL << 38;
 
-// 32-bit words of the parts of a grid's scratch, in the order they lie there
-struct PartialWords {
-  size_t acc, stat, header;  // [2 ctas][g * d] accumulators, [2 ctas][g] twice (m, l), [ctas][4]
-  __host__ __device__ constexpr PartialWords(size_t ctas, size_t g, size_t d) : acc(2 * ctas * g * d), stat(2 * ctas * g), header(4 * ctas) {}
-  __host__ __device__ constexpr size_t all() const { return acc + 2 * stat + header; }
-};
+// 32-bit words of scratch per CTA: two accumulators, twice two statistics, a header
+constexpr size_t partial_words(size_t g, size_t d) { return 2 * g * d + 2 * (2 * g) + 4; }
 template <int G, int D>
 struct Partials {  // scratch of a grid of `ctas`
+  static constexpr size_t kAcc = 2 * G * D, kStat = 2 * G, kHeader = 4;  // words per CTA
+  static_assert(kAcc + 2 * kStat + kHeader == partial_words(G, D), "what the size function asks for is what is laid out here");
   float* acc;      // [2 ctas][G * D]
   float* m;        // [2 ctas][G]
   float* l;        // [2 ctas][G]
-  int* header;     // [ctas][4]: token, KV head, CTA that ends the item that CTA b begins; token < 0: none
-  __device__ Partials(float* base, unsigned ctas) {
-    const PartialWords words(ctas, G, D);
-    acc = base, m = acc + words.acc, l = m + words.stat, header = reinterpret_cast<int*>(l + words.stat);
+  int* header;     // [ctas][kHeader]: token, KV head, CTA that ends the item that CTA b begins; token < 0: none
+  __device__ Partials(float* base, int ctas) {
+    acc = base;
+    m = acc + kAcc * ctas;
+    l = m + kStat * ctas;
+    header = reinterpret_cast<int*>(l + kStat * ctas);
   }
 };
 
@@ -969,7 +969,7 @@ extern "C" size_t xdk_paged_decode_attention_scratch_bytes(int64_t tokens, int64
   if (head_dim != 64 && head_dim != 128 && head_dim != 256) return 0;
   const int g = static_cast<int>(q_heads / kv_heads);
   const int ctas = even_grid(tokens, kv_heads, head_dim, context_hint, dtype == XDK_F32 ? 4 : 2, g);
-  return PartialWords(ctas, g, head_dim).all() * 4;
+  return ctas * partial_words(g, head_dim) * 4;
 }
 
 extern "C" int xdk_paged_decode_attention_ws(const void* q, const void* k_cache, const void* v_cache, const int64_t* positions,
