@@ -137,16 +137,17 @@ __device__ __forceinline__ U4 ld_cached16(const void* p) {
 }
 // Loads of what the preceding kernel may have written: activations, caches, index tensors.  A load through the read-only path
 // (ld_cached16, ld_stream16, __ldg, or a plain one through a const __restrict__ pointer) counts as invariant, and the compiler
-// may move it in front of pdl_wait(); these stay behind it, as does a plain load through a pointer without __restrict__.
+// may move it in front of pdl_wait(); these stay behind it, as does a plain load through a pointer without __restrict__.  (For
+// what this kernel does not write itself: they are ordered with other volatile statements, not with its stores.)
 __device__ __forceinline__ U4 ld_ordered16(const void* p) {
   U4 v;
-  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
 __device__ __forceinline__ U4 ld_ordered_stream16(const void* p) {  // each byte is used once: not kept in L1
   U4 v;
   asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
 __device__ __forceinline__ float4 ld_stream_f4(const float* p) {
