@@ -309,7 +309,7 @@ struct StageV {  // whether a warp's V rows are staged in shared memory beside i
 };
 
 template <typename T, int G, int D>
-__global__ void __launch_bounds__(kAttnThreads)
+__global__ void __launch_bounds__(kAttnThreads, D <= 128 ? 3 : 1)  // what its shared memory leaves room for
 paged_decode_attention_kernel(const T* q, const T* k_cache, const T* v_cache,
                               const __grid_constant__ PeerOut out, const __grid_constant__ AttnArgs a, int splits) {
   constexpr int E = 16 / sizeof(T);   // elements per 16-byte piece
