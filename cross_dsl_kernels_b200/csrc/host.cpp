@@ -1,12 +1,12 @@
 // The eager calls of ops.py and w4a16.py in native code: check the tensors, allocate the outputs, launch.
 //
 // A decode step called eagerly is bound by the host: the checks and the ctypes call of one op took 17 - 75 us of Python,
-// several times the kernel.  Here they take 5 (a BF16 norm of 16 x 4096: 18.7 -> 6.2 us a call; an append of few tokens:
-// 76 -> 5.3; two eager decode layers of 4 tokens, 14 calls: 501 -> 123).  Each function here takes the arguments of the Python op by
-// position, repeats the op's
-// conditions on the tensors' metadata, and launches through the same C ABI entry point on torch's current stream.  It
-// takes the ordinary call only: where a condition fails, or an argument has another form than the ordinary one (a tensor
-// subclass, an odd type), it returns None and the Python function decides -- and words the error -- as before.
+// several times the kernel.  Here they take 5 (a BF16 norm of 16 x 4096: 18.7 -> 5.9 us a call; an append of few tokens:
+// 76 -> 5.3; two eager decode layers of 4 tokens, 14 calls: 492 -> 120).  Each function here takes the arguments of the
+// Python op by position, repeats the op's conditions on the tensors' metadata, and launches through the same C ABI entry
+// point on torch's current stream.  It takes the ordinary call only: where a condition fails, or an argument has another
+// form than the ordinary one (a tensor subclass, an odd type), it returns None and the Python function decides -- and words
+// the error -- as before.
 // Outputs come from torch's allocator (at::empty), so streams, graph capture and dispatch modes see what they saw.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
